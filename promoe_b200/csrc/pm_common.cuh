@@ -51,6 +51,12 @@ constexpr int kMaxChunkRows = 64;   // token rows per chunk (8 MMA n-tiles)
 constexpr int kSplitMaxRows = 16;   // launches whose chunks all fit use the split-K decode kernel,
 constexpr int kSplitTileGu = 16;    // whose tiles are 16 gate+up rows
 constexpr int kSplitTileDn = 32;    // or 32 down rows
+// Most rows of a bf16 group that still runs as 16-row chunks of the split-K kernel; above, one tensor-core
+// tile streams its weights once. Measured on a layer of 64 tokens x top-8 over experts of 1-40 rows
+// (hidden 3584, inter 2560, shared 20480): FFN 796 us with this line at 32, 874 us at 64; a prompt of 777
+// tokens x top-4 over 60 experts: 326 us at 32, 382 us at 64. (At 16 a decode batch of 32 loses 45 us: its
+// shared expert alone then costs a launch pair of its own.)
+constexpr int kSplitChunkedMaxRows = 32;
 
 // Kernel launchers (defined in the .cu files). All take the caller's stream.
 cudaError_t launch_gate_topk(const __nv_bfloat16* x, const __nv_bfloat16* w_gate, const float* bias,
@@ -155,22 +161,27 @@ cudaError_t launch_combine(const float* yexp, const int32_t* pos, const float* t
                            int k, int R, int n_shared, const float* shared_scale,
                            __nv_bfloat16* y, cudaStream_t s);
 
-// ---- prefill path (tcgen05) ---------------------------------------------------------------------
-// Tensor maps of one launch pair: token rows (expert-sorted x, intermediate h), the slab (3-D:
-// k, weight row, cache line) per projection, and the layer's shared expert (2-D).
+// ---- tensor-core path (tcgen05) ------------------------------------------------------------------
+// Tensor maps of one launch pair. Token rows (expert-sorted x, intermediate h): one map per box height
+// 16, 32, 64, 128, so that a tile's rows arrive in as few boxes as possible (a box costs the copy engine
+// about as much as 16 KB of data). Weights: routed experts through maps over the whole slab whose last
+// coordinate is the cache line, the layer's shared expert through maps of its own. The gate/up maps
+// see both matrices as (k, row in block of 16, matrix, block, line), so that one box of 4 blocks brings
+// 64 gate and 64 up rows, alternating in blocks of 16; the matrix with the lower address comes first.
 struct TcMaps {
-  CUtensorMap a_x, a_h, slab_gate, slab_up, slab_down, sh_gate, sh_up, sh_down;
+  CUtensorMap a_x[4], a_h[4], slab_gu, slab_down, sh_gu, sh_down;
+  int32_t slab_up_first, sh_up_first;
 };
 struct TcGroup {
   int32_t row_start, row_count, inter;
   int32_t line;  // global cache line of the expert, -1 = the shared expert
 };
-struct TcTile {
-  int32_t group, m0, n0, pad;
-};
-cudaError_t launch_prefill_ffn(const TcMaps& maps, const TcGroup* groups_dev, const TcTile* tiles_gu_dev, int n_gu,
-                               const TcTile* tiles_dn_dev, int n_dn, int hidden, __nv_bfloat16* hbuf, int ld_h,
-                               float* yexp, int32_t* err_dev, cudaStream_t s, cudaEvent_t mid_event);
+constexpr int kTcMaxN = 256;       // token rows per tile
+constexpr int kMaxTcGroups = 264;  // groups of one launch pair (every expert and the shared one)
+// tiles_gu / tiles_dn: tiles of the two launches (tc_tile_count), which bound their grids.
+cudaError_t launch_prefill_ffn(const TcMaps& maps, const TcGroup* groups_dev, int n_groups, int tiles_gu, int tiles_dn,
+                               int hidden, __nv_bfloat16* hbuf, int ld_h, float* yexp, int32_t* err_dev, cudaStream_t s,
+                               cudaEvent_t mid_event);
 
 // out[r] = index of the r-th best of scores[0 .. width) (descending, ties to the lower index), r < n.
 cudaError_t launch_rank_topn(const float* scores, int width, int n, int32_t* out, cudaStream_t s);

@@ -153,11 +153,8 @@ int ensure_workspace(pm_ctx* c, int T, const pm_layer_weights& w) {
   const int Is = std::max(w.shared_inter, c->ws_inter_shared);
   size_t o_res = take((size_t)(kMaxFusedGroups + 1) * 4);
   size_t o_xp = take(rows * H * 2);
-  {
-    const size_t m_tiles = rows / 128 + (size_t)E + 2;
-    c->tc_plan_cap = 16 * ((size_t)E + 2) + 16 * m_tiles * ((size_t)(std::max(I, Is) + 127) / 128 + (size_t)(H + 127) / 128) + 1024 +
-                     768 * ((size_t)E + 2);  // three 256-byte roundings per segment, at most one segment per expert
-  }
+  // the groups of every expert and the shared one, and a 256-byte rounding per segment (at most one per expert)
+  c->tc_plan_cap = (sizeof(TcGroup) + 256) * ((size_t)E + 2);
   size_t o_tcp = take(c->tc_plan_cap);
   c->perm_scratch_ints = (R / 4096 + 2) * (size_t)E;
   size_t o_ps = take(c->perm_scratch_ints * 4);
@@ -538,8 +535,8 @@ struct PendingForward {
 
 namespace {
 
-// Prefill-size segment on the tcgen05 path: gather the token rows once per layer call, plan the
-// 128 x 128 tiles, upload groups and tiles, launch the gate/up and the down kernel.
+// Segment on the tcgen05 path: gather the token rows once per layer call, upload the groups, launch
+// the gate/up and the down kernel.
 int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows,
                      cudaStream_t s, bool q4 = false) {
   if (!c->xperm_ready) {
@@ -578,17 +575,13 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
     groups.push_back(TcGroup{g.row_start, g.row_count, g.inter, line});
   }
   const TcMaps& maps = q4 ? c->tc_maps_q4 : c->tc_maps;
-  std::vector<TcTile> gu, dn;
-  tc_plan(groups, w.hidden, &gu, &dn);
-  const size_t g_bytes = align_up(groups.size() * sizeof(TcGroup), 256);
-  const size_t gu_bytes = align_up(gu.size() * sizeof(TcTile), 256), dn_bytes = align_up(dn.size() * sizeof(TcTile), 256);
-  const size_t total = g_bytes + gu_bytes + dn_bytes;
+  int tiles_gu = 0, tiles_dn = 0;
+  for (const TcGroup& g : groups) tc_tile_count(g, w.hidden, &tiles_gu, &tiles_dn);
+  const size_t total = align_up(groups.size() * sizeof(TcGroup), 256);
   if (c->tc_plan_used + total > c->tc_plan_cap) return fail(PM_ERR_STATE, "prefill plan buffer overflow");
   unsigned char* h = c->h_tc_plan + c->tc_plan_used;
   unsigned char* d = c->d_tc_plan + c->tc_plan_used;
   std::memcpy(h, groups.data(), groups.size() * sizeof(TcGroup));
-  std::memcpy(h + g_bytes, gu.data(), gu.size() * sizeof(TcTile));
-  std::memcpy(h + g_bytes + gu_bytes, dn.data(), dn.size() * sizeof(TcTile));
   PM_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, s));
   c->tc_plan_used += total;
   pm_ctx::FfnSample sample{};
@@ -602,9 +595,8 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
     }
     PM_CUDA(cudaEventRecord(sample.e0, s));
   }
-  PM_CUDA(launch_prefill_ffn(maps, (const TcGroup*)d, (const TcTile*)(d + g_bytes), (int)gu.size(),
-                             (const TcTile*)(d + g_bytes + gu_bytes), (int)dn.size(), w.hidden, c->d_hbuf, c->ws_inter,
-                             c->d_yexp, c->d_tc_err, s, c->profile_ffn ? sample.e1 : nullptr));
+  PM_CUDA(launch_prefill_ffn(maps, (const TcGroup*)d, (int)groups.size(), tiles_gu, tiles_dn, w.hidden, c->d_hbuf,
+                             c->ws_inter, c->d_yexp, c->d_tc_err, s, c->profile_ffn ? sample.e1 : nullptr));
   if (c->profile_ffn) {
     PM_CUDA(cudaEventRecord(sample.e2, s));
     c->ffn_samples.push_back(sample);
@@ -654,18 +646,18 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
   }
   // Groups with many rows go to the tensor cores; the others stay on the split-K tiles, which stream
   // the weights faster when there are only a few rows to use them for (a large decode batch has both
-  // kinds in one layer call). uint4 groups change over later: expanding an expert to bf16 costs more
-  // than re-reading its packed weights a few times.
+  // kinds in one layer call). Up to kSplitChunkedMaxRows rows a group runs as chunks of 16 rows through the
+  // split-K tiles (its weights are read once from HBM and again from L2 for the later chunks). uint4
+  // groups change over later: expanding an expert to bf16 costs more than re-reading its packed
+  // weights a few times.
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
-  // Up to kMaxChunkRows rows a group runs as chunks of 16 rows through the split-K tiles (its weights
-  // are read once from HBM and again from L2 for the later chunks): a 128-row tensor-core tile would be
-  // mostly padding there, and a few such groups alone give that kernel too few CTAs to stream from.
-  const int most_small = w.quant4 ? kQ4ExpandMinRows - 1 : kMaxChunkRows;
+  const bool tc_shared_ok = tc_shared_usable(w);
+  const int most_small = w.quant4 ? kQ4ExpandMinRows - 1 : kSplitChunkedMaxRows;
   Segment big;
   if (tc_ok) {
     size_t keep = 0;
     for (size_t i = 0; i < seg->groups.size(); ++i) {
-      if (seg->groups[i].row_count > most_small) {
+      if (seg->groups[i].row_count > most_small && (seg->group_line[i] >= 0 || tc_shared_ok)) {
         big.groups.push_back(seg->groups[i]);
         big.group_line.push_back(seg->group_line[i]);
       } else {

@@ -133,9 +133,9 @@ struct pm_ctx {
   size_t h_stage_bytes = 0;
 
   // ---- prefill (tcgen05) path ---------------------------------------------------------------------
-  bool tc_prefill = true;             // use it for experts with more than 64 rows in a call
+  bool tc_prefill = true;             // use it for experts with more than kSplitChunkedMaxRows rows in a call
   __nv_bfloat16* d_xperm = nullptr;   // expert-sorted copy of the token rows [rows, hidden]
-  unsigned char* d_tc_plan = nullptr; // groups + tiles of the segments of one layer call
+  unsigned char* d_tc_plan = nullptr; // groups of the segments of one layer call
   unsigned char* h_tc_plan = nullptr; // pinned staging of the same
   size_t tc_plan_cap = 0, tc_plan_used = 0;
   int32_t* d_perm_scratch = nullptr;  // per-chunk expert counts of the multi-CTA permutation
@@ -234,9 +234,10 @@ void rt_mark_dirty(pm_ctx* c, const std::vector<Action>& actions);
 int rt_profile_collect(pm_ctx* c);
 bool tc_prefill_usable(const pm_ctx* c, const pm_layer_weights& w);
 bool tc_prefill_usable_q4(const pm_ctx* c, const pm_layer_weights& w);
+bool tc_shared_usable(const pm_layer_weights& w);  // one tensor map can span the shared gate and up matrices
 int tc_build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m);
 // Same with the routed experts' bf16 weights in `slab` (gate, up, down back to back in every line).
 int tc_build_maps_q4(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m);
-void tc_plan(const std::vector<TcGroup>& groups, int hidden, std::vector<TcTile>* gu, std::vector<TcTile>* dn);
+void tc_tile_count(const TcGroup& g, int hidden, int* gu, int* dn);  // adds the group's tiles
 
 }  // namespace pm

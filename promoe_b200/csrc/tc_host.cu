@@ -25,12 +25,12 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// bf16 tensor, innermost dimension k: box = 64 k x 128 rows (x 1 line), 128-byte swizzle, zero fill.
-int encode(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes) {
+// bf16 tensor, innermost dimension k, 64 k (128 bytes) wide boxes, 128-byte swizzle, zero fill.
+int encode(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
+           const cuuint32_t* box) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return fail(PM_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
-  cuuint32_t box[3] = {64, 128, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides_bytes,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -38,10 +38,35 @@ int encode(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims,
   return PM_OK;
 }
 
-int encode_2d(CUtensorMap* map, const void* base, uint64_t k, uint64_t rows, uint64_t pitch_elems) {
+// Token rows: one map per box height.
+int encode_rows(CUtensorMap (&maps)[4], const void* base, uint64_t k, uint64_t rows, uint64_t pitch_elems) {
   cuuint64_t dims[2] = {k, rows};
   cuuint64_t strides[1] = {pitch_elems * 2};
-  return encode(map, base, 2, dims, strides);
+  for (int i = 0; i < 4; ++i) {
+    cuuint32_t box[2] = {64, 16u << i};
+    int rc = encode(&maps[i], base, 2, dims, strides, box);
+    if (rc != PM_OK) return rc;
+  }
+  return PM_OK;
+}
+
+// Gate and up projections [inter, hidden] of `lines` experts `stride` bytes apart, as one map.
+int encode_gate_up(CUtensorMap* map, int32_t* up_first, const unsigned char* gate, const unsigned char* up, uint64_t hidden,
+                   uint64_t inter, uint64_t stride, uint64_t lines) {
+  *up_first = up < gate;
+  const unsigned char* base = std::min(gate, up);
+  const uint64_t apart = (uint64_t)(std::max(gate, up) - base);
+  cuuint64_t dims[5] = {hidden, 16, 2, inter / 16, lines};
+  cuuint64_t strides[4] = {hidden * 2, apart, hidden * 32, stride};
+  cuuint32_t box[5] = {64, 16, 2, 4, 1};
+  return encode(map, base, 5, dims, strides, box);
+}
+
+int encode_down(CUtensorMap* map, const void* down, uint64_t hidden, uint64_t inter, uint64_t stride, uint64_t lines) {
+  cuuint64_t dims[3] = {inter, hidden, lines};
+  cuuint64_t strides[2] = {inter * 2, stride};
+  cuuint32_t box[3] = {64, 128, 1};
+  return encode(map, down, 3, dims, strides, box);
 }
 
 }  // namespace
@@ -57,43 +82,38 @@ bool tc_prefill_usable_q4(const pm_ctx* c, const pm_layer_weights& w) {
   return w.hidden % 128 == 0 && w.inter % 128 == 0 && w.shared_inter % 64 == 0;
 }
 
+// Strides of a tensor map stay below 2^40 bytes: matrices further apart (memory of different allocators)
+// leave the shared expert on the other kernels.
+bool tc_shared_usable(const pm_layer_weights& w) {
+  const uintptr_t g = (uintptr_t)w.shared_w_gate, u = (uintptr_t)w.shared_w_up;
+  return (g > u ? g - u : u - g) < ((uintptr_t)1 << 40);
+}
+
 namespace {
 
 // Maps of the token rows, of a slab of bf16 expert lines (`lines` lines `stride` bytes apart, the
 // three matrices at the given addresses of line 0) and of the layer's shared expert.
 int build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, const unsigned char* gate0,
                const unsigned char* up0, const unsigned char* down0, uint64_t stride, uint64_t lines, TcMaps* m) {
-  const uint64_t H = w.hidden, I = w.inter;
-  int rc = encode_2d(&m->a_x, c->d_xperm, H, (uint64_t)rows_cap, H);
+  const uint64_t H = w.hidden, I = w.inter, Is = w.shared_inter;
+  int rc = encode_rows(m->a_x, c->d_xperm, H, (uint64_t)rows_cap, H);
   if (rc != PM_OK) return rc;
-  rc = encode_2d(&m->a_h, c->d_hbuf, (uint64_t)c->ws_inter, (uint64_t)rows_cap, (uint64_t)c->ws_inter);
+  rc = encode_rows(m->a_h, c->d_hbuf, (uint64_t)c->ws_inter, (uint64_t)rows_cap, (uint64_t)c->ws_inter);
   if (rc != PM_OK) return rc;
-  {
-    cuuint64_t dims[3] = {H, I, lines};
-    cuuint64_t strides[2] = {H * 2, (cuuint64_t)stride};
-    rc = encode(&m->slab_gate, gate0, 3, dims, strides);
+  rc = encode_gate_up(&m->slab_gu, &m->slab_up_first, gate0, up0, H, I, stride, lines);
+  if (rc != PM_OK) return rc;
+  rc = encode_down(&m->slab_down, down0, H, I, stride, lines);
+  if (rc != PM_OK) return rc;
+  if (Is > 0 && tc_shared_usable(w)) {  // one "line"; its stride is never used but has to be a valid one
+    rc = encode_gate_up(&m->sh_gu, &m->sh_up_first, (const unsigned char*)w.shared_w_gate, (const unsigned char*)w.shared_w_up, H,
+                        Is, H * 32, 1);
     if (rc != PM_OK) return rc;
-    rc = encode(&m->slab_up, up0, 3, dims, strides);
-    if (rc != PM_OK) return rc;
-  }
-  {
-    cuuint64_t dims[3] = {I, H, lines};
-    cuuint64_t strides[2] = {I * 2, (cuuint64_t)stride};
-    rc = encode(&m->slab_down, down0, 3, dims, strides);
-    if (rc != PM_OK) return rc;
-  }
-  if (w.shared_inter > 0) {
-    const uint64_t Is = w.shared_inter;
-    rc = encode_2d(&m->sh_gate, w.shared_w_gate, H, Is, H);
-    if (rc != PM_OK) return rc;
-    rc = encode_2d(&m->sh_up, w.shared_w_up, H, Is, H);
-    if (rc != PM_OK) return rc;
-    rc = encode_2d(&m->sh_down, w.shared_w_down, Is, H, Is);
+    rc = encode_down(&m->sh_down, w.shared_w_down, H, Is, Is * 2, 1);
     if (rc != PM_OK) return rc;
   } else {  // never dereferenced: any valid map keeps the parameter well formed
-    m->sh_gate = m->slab_gate;
-    m->sh_up = m->slab_up;
+    m->sh_gu = m->slab_gu;
     m->sh_down = m->slab_down;
+    m->sh_up_first = 0;
   }
   return PM_OK;
 }
@@ -111,18 +131,11 @@ int tc_build_maps_q4(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps*
                     (uint64_t)c->q4_scratch_stride, (uint64_t)c->q4_scratch_lines, m);
 }
 
-// Tiles of one segment: every 128-row block of every group times every 128-column block of the
-// gate/up projections and every 256-column block of the down projection.
-void tc_plan(const std::vector<TcGroup>& groups, int hidden, std::vector<TcTile>* gu, std::vector<TcTile>* dn) {
-  gu->clear();
-  dn->clear();
-  for (int g = 0; g < (int)groups.size(); ++g) {
-    const TcGroup& grp = groups[g];
-    for (int m0 = 0; m0 < grp.row_count; m0 += 128) {
-      for (int n0 = 0; n0 < grp.inter; n0 += 128) gu->push_back(TcTile{g, m0, n0, 0});
-      for (int n0 = 0; n0 < hidden; n0 += 256) dn->push_back(TcTile{g, m0, n0, 0});
-    }
-  }
+// Tiles of one group: token tiles of at most kTcMaxN rows times blocks of 128 gate/up rows or 256 down rows.
+void tc_tile_count(const TcGroup& g, int hidden, int* gu, int* dn) {
+  const int n = (g.row_count + kTcMaxN - 1) / kTcMaxN;
+  *gu += n * ((g.inter + 127) / 128);
+  *dn += n * ((hidden + 255) / 256);
 }
 
 }  // namespace pm
