@@ -150,10 +150,6 @@ inline bool ffn_launch_is_fused(const FfnPlanInfo& info, int quant4) {
   return info.max_rows <= kSplitMaxRows && info.n_desc <= (quant4 ? kMaxFusedGroupsQ4 : kMaxFusedGroups);
 }
 
-// uint4 group-128 matrix [rows, K] (packed words + {scale, zero} fp16 pairs) -> bf16 [rows, K].
-cudaError_t launch_dequant_q4(const void* packed, const void* scale_zero, int rows, int K, __nv_bfloat16* out,
-                              cudaStream_t s);
-
 cudaError_t launch_gather_rows(const void* src, const int32_t* index, int n_rows, size_t row_bytes, void* dst,
                                cudaStream_t s);
 
@@ -178,10 +174,21 @@ struct TcGroup {
 };
 constexpr int kTcMaxN = 256;       // token rows per tile
 constexpr int kMaxTcGroups = 264;  // groups of one launch pair (every expert and the shared one)
-// tiles_gu / tiles_dn: tiles of the two launches (tc_tile_count), which bound their grids.
-cudaError_t launch_prefill_ffn(const TcMaps& maps, const TcGroup* groups_dev, int n_groups, int tiles_gu, int tiles_dn,
-                               int hidden, __nv_bfloat16* hbuf, int ld_h, float* yexp, int32_t* err_dev, cudaStream_t s,
-                               cudaEvent_t mid_event);
+struct TcLaunch {
+  const TcMaps* maps;
+  const TcGroup* groups_dev;
+  int n_groups, max_rows;      // groups, rows of the largest
+  int tiles_gu, tiles_dn;      // tiles of the two launches (tc_tile_count), which bound their grids
+  int hidden, ld_h;
+  __nv_bfloat16* hbuf;
+  float* yexp;
+  int32_t* err_dev;
+  // uint4 experts (scale_base non-null; the slab maps then describe the packed matrices): {scale, zero} pairs
+  // of cache line l at scale_base + l * scale_stride + the projection's offset
+  const unsigned char* scale_base = nullptr;
+  size_t scale_stride = 0, scale_gate = 0, scale_up = 0, scale_down = 0;
+};
+cudaError_t launch_prefill_ffn(const TcLaunch& a, cudaStream_t s, cudaEvent_t mid_event);
 
 // out[r] = index of the r-th best of scores[0 .. width) (descending, ties to the lower index), r < n.
 cudaError_t launch_rank_topn(const float* scores, int width, int n, int32_t* out, cudaStream_t s);

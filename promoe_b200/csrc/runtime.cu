@@ -535,46 +535,30 @@ struct PendingForward {
 
 namespace {
 
-// Segment on the tcgen05 path: gather the token rows once per layer call, upload the groups, launch
-// the gate/up and the down kernel.
+// Groups on the tcgen05 path: gather the token rows once per layer call, upload the groups, launch the
+// gate/up and the down kernel. All groups are of one kind: uint4 experts (q4), which the kernel expands
+// to bf16 on their way into shared memory, or bf16 (experts and the shared expert).
 int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows,
-                     cudaStream_t s, bool q4 = false) {
+                     cudaStream_t s, bool q4) {
   if (!c->xperm_ready) {
     PM_CUDA(launch_gather_rows(x, c->d_row_token, n_rows, (size_t)w.hidden * 2, c->d_xperm, s));
     c->kernel_launches += 1;
     c->xperm_ready = true;
   }
-  if (q4) {
-    if (!c->tc_maps_q4_ready) {
-      int rc = tc_build_maps_q4(c, w, c->ws_tokens * (c->ws_topk + 1), &c->tc_maps_q4);
-      if (rc != PM_OK) return rc;
-      c->tc_maps_q4_ready = true;
-    }
-  } else if (!c->tc_maps_ready) {
+  if (!c->tc_maps_ready) {
     int rc = tc_build_maps(c, w, c->ws_tokens * (c->ws_topk + 1), &c->tc_maps);
     if (rc != PM_OK) return rc;
     c->tc_maps_ready = true;
   }
   std::vector<TcGroup> groups;
+  int max_rows = 0;
   for (size_t i = 0; i < seg->groups.size(); ++i) {
     const pm_ffn_group& g = seg->groups[i];
     if (g.row_count <= 0) continue;
-    int line = seg->group_line[i];
-    if (q4 && line >= 0) {
-      // expand the expert's packed matrices into scratch line n (stream order keeps the line's earlier
-      // readers ahead of this write); the tensor-core kernels then read bf16 as for any other expert
-      line = (int)groups.size();
-      unsigned char* dst = c->q4_scratch + (size_t)line * c->q4_scratch_stride;
-      const size_t mat = (size_t)w.inter * w.hidden * 2;
-      PM_CUDA(launch_dequant_q4(g.w_gate, g.q_gate, w.inter, w.hidden, (__nv_bfloat16*)dst, s));
-      PM_CUDA(launch_dequant_q4(g.w_up, g.q_up, w.inter, w.hidden, (__nv_bfloat16*)(dst + mat), s));
-      PM_CUDA(launch_dequant_q4(g.w_down, g.q_down, w.hidden, w.inter, (__nv_bfloat16*)(dst + 2 * mat), s));
-      c->kernel_launches += 3;
-      c->q4_expanded += 1;
-    }
-    groups.push_back(TcGroup{g.row_start, g.row_count, g.inter, line});
+    groups.push_back(TcGroup{g.row_start, g.row_count, g.inter, seg->group_line[i]});
+    max_rows = std::max(max_rows, g.row_count);
   }
-  const TcMaps& maps = q4 ? c->tc_maps_q4 : c->tc_maps;
+  if (q4) c->q4_expanded += (int64_t)groups.size();
   int tiles_gu = 0, tiles_dn = 0;
   for (const TcGroup& g : groups) tc_tile_count(g, w.hidden, &tiles_gu, &tiles_dn);
   const size_t total = align_up(groups.size() * sizeof(TcGroup), 256);
@@ -590,13 +574,32 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
     PM_CUDA(cudaEventCreate(&sample.e1));
     PM_CUDA(cudaEventCreate(&sample.e2));
     for (const TcGroup& g : groups) {
-      sample.bytes_gu += 4ll * g.inter * w.hidden;
-      sample.bytes_dn += 2ll * g.inter * w.hidden;
+      const int64_t mat = (int64_t)g.inter * w.hidden, one = q4 ? mat / 2 + mat / 128 * 4 : mat * 2;
+      sample.bytes_gu += 2 * one;
+      sample.bytes_dn += one;
     }
     PM_CUDA(cudaEventRecord(sample.e0, s));
   }
-  PM_CUDA(launch_prefill_ffn(maps, (const TcGroup*)d, (int)groups.size(), tiles_gu, tiles_dn, w.hidden, c->d_hbuf,
-                             c->ws_inter, c->d_yexp, c->d_tc_err, s, c->profile_ffn ? sample.e1 : nullptr));
+  TcLaunch a{};
+  a.maps = &c->tc_maps;
+  a.groups_dev = (const TcGroup*)d;
+  a.n_groups = (int)groups.size();
+  a.max_rows = max_rows;
+  a.tiles_gu = tiles_gu;
+  a.tiles_dn = tiles_dn;
+  a.hidden = w.hidden;
+  a.ld_h = c->ws_inter;
+  a.hbuf = c->d_hbuf;
+  a.yexp = c->d_yexp;
+  a.err_dev = c->d_tc_err;
+  if (q4) {
+    a.scale_base = c->slab;
+    a.scale_stride = c->line_stride;
+    a.scale_gate = c->param_offset[c->role_qgate];
+    a.scale_up = c->param_offset[c->role_qup];
+    a.scale_down = c->param_offset[c->role_qdown];
+  }
+  PM_CUDA(launch_prefill_ffn(a, s, c->profile_ffn ? sample.e1 : nullptr));
   if (c->profile_ffn) {
     PM_CUDA(cudaEventRecord(sample.e2, s));
     c->ffn_samples.push_back(sample);
@@ -606,32 +609,70 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
   return PM_OK;
 }
 
-// Rows per expert from which uint4 experts are expanded to bf16 and run on the tensor
-// cores: below it, re-reading the packed weights once per 16 rows is cheaper than writing and
-// re-reading four times as many bf16 bytes.
-constexpr int kQ4ExpandMinRows = 64;
+// Whether the uint4 experts of a segment go to the tensor cores. The split-K kernel's time follows the 16-row
+// chunks (it unpacks the weights once per chunk), the tensor-core kernel's the experts (it expands them
+// once per 256 rows): measured on 8 experts of 4096 x 14336, 49 us a chunk of 9-16 rows against 75 us an
+// expert. All of them go one way, because a launch pair for a few experts leaves most SMs idle in its down
+// pass (105 us for one expert, 200 us for all 8). Layer calls of 64 / 128 / 512 tokens x top-2: 595 / 985 / 1505 us
+// when each expert from 64 rows on was expanded to a bf16 slab first, 560 / 597 / 653 us now.
+bool q4_prefers_tc(const Segment& seg) {
+  int groups = 0, chunks = 0;
+  for (size_t i = 0; i < seg.groups.size(); ++i)
+    if (seg.group_line[i] >= 0 && seg.groups[i].row_count > 0) {
+      ++groups;
+      chunks += (seg.groups[i].row_count + kSplitMaxRows - 1) / kSplitMaxRows;
+    }
+  return 2 * chunks > 3 * groups;
+}
 
-// The bf16 scratch slab for `n` expanded experts (grown on demand, at least one line per expert of
-// a layer). False if the device cannot provide it: the caller then stays on the split-K tiles.
-bool q4_scratch_ready(pm_ctx* c, const pm_layer_weights& w, int n) {
-  const size_t stride = align_up((size_t)3 * w.inter * w.hidden * 2, 256);
-  const size_t lines = (size_t)std::max(n, c->cfg.num_expert);
-  if (c->q4_scratch != nullptr && c->q4_scratch_stride == stride && c->q4_scratch_lines >= lines) return true;
-  if (c->q4_scratch != nullptr) {
-    cudaDeviceSynchronize();  // earlier launches may still read the old slab
-    cudaFree(c->q4_scratch);
-    c->q4_scratch = nullptr;
-    c->q4_scratch_lines = 0;
+// Groups on the split-K / staged kernels: plan them, upload the plan, launch. All groups are of one kind
+// (quant4, or bf16).
+int flush_groups_split(pm_ctx* c, const std::vector<pm_ffn_group>& groups, bool quant4, bool tc_ok, const pm_layer_weights& w,
+                       const __nv_bfloat16* x, size_t* desc_used, cudaStream_t s) {
+  FfnPlanInfo info;
+  // without the tensor-core path (shapes it cannot tile) larger groups stay in 64-row chunks for the staged kernel
+  const int chunk_rows = (quant4 || w.quant4 || tc_ok) ? kSplitMaxRows : kMaxChunkRows;
+  int rc = plan_groups_size(groups.data(), (int)groups.size(), w.hidden, &info, chunk_rows);
+  if (rc != PM_OK) return rc;
+  if (*desc_used + info.blob_bytes() > c->plan_cap) return fail(PM_ERR_STATE, "launch plan buffer overflow");
+  Stage st = stage_of(c);
+  rc = plan_groups_into(groups.data(), (int)groups.size(), w.hidden, st.plan + *desc_used,
+                        c->plan_cap - *desc_used, &info, chunk_rows);
+  if (rc != PM_OK) return rc;
+  PM_CUDA(cudaMemcpyAsync(c->d_plan + *desc_used, st.plan + *desc_used, info.blob_bytes(), cudaMemcpyHostToDevice, s));
+  pm_ctx::FfnSample sample{};
+  if (c->profile_ffn) {
+    auto take_event = [&](cudaEvent_t* e) -> cudaError_t {
+      if (!c->ffn_event_pool.empty()) {
+        *e = c->ffn_event_pool.back();
+        c->ffn_event_pool.pop_back();
+        return cudaSuccess;
+      }
+      return cudaEventCreate(e);
+    };
+    sample.fused = ffn_launch_is_fused(info, quant4);
+    PM_CUDA(take_event(&sample.e0));
+    if (!sample.fused) PM_CUDA(take_event(&sample.e1));
+    PM_CUDA(take_event(&sample.e2));
+    for (const pm_ffn_group& g : groups) {
+      int64_t mat = (int64_t)g.inter * w.hidden;
+      // uint4: half a byte per weight plus one fp16 {scale, zero} pair per 128 weights
+      int64_t one = quant4 ? mat / 2 + mat / 128 * 4 : mat * 2;
+      sample.bytes_gu += 2 * one;
+      sample.bytes_dn += one;
+    }
+    PM_CUDA(cudaEventRecord(sample.e0, s));
   }
-  if (cudaMalloc((void**)&c->q4_scratch, stride * lines) != cudaSuccess) {
-    cudaGetLastError();
-    c->q4_scratch = nullptr;
-    return false;
+  PM_CUDA(launch_swiglu_ffn(c->d_plan + *desc_used, info, quant4, x, w.hidden, c->d_row_token, c->d_hbuf,
+                            c->ws_inter, c->d_yexp, s, (c->profile_ffn && !sample.fused) ? sample.e1 : nullptr,
+                            c->d_tc_err));
+  if (c->profile_ffn) {
+    PM_CUDA(cudaEventRecord(sample.e2, s));
+    c->ffn_samples.push_back(sample);
   }
-  c->q4_scratch_stride = stride;
-  c->q4_scratch_lines = lines;
-  c->tc_maps_q4_ready = false;
-  return true;
+  c->kernel_launches += ffn_launch_is_fused(info, quant4) ? 1 : 2;
+  *desc_used += align_up(info.blob_bytes(), 256);
+  return PM_OK;
 }
 
 int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows,
@@ -646,20 +687,21 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
   }
   // Groups with many rows go to the tensor cores; the others stay on the split-K tiles, which stream
   // the weights faster when there are only a few rows to use them for (a large decode batch has both
-  // kinds in one layer call). Up to kSplitChunkedMaxRows rows a group runs as chunks of 16 rows through the
-  // split-K tiles (its weights are read once from HBM and again from L2 for the later chunks). uint4
-  // groups change over later: expanding an expert to bf16 costs more than re-reading its packed
-  // weights a few times.
+  // kinds in one layer call). Below the line a group runs as chunks of 16 rows through the split-K
+  // tiles: its weights are read once from HBM and again from L2 for the later chunks.
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
   const bool tc_shared_ok = tc_shared_usable(w);
-  const int most_small = w.quant4 ? kQ4ExpandMinRows - 1 : kSplitChunkedMaxRows;
-  Segment big;
+  const bool q4_tc = w.quant4 && tc_ok && q4_prefers_tc(*seg);
+  Segment big, big_shared;  // the shared expert of a uint4 layer is bf16: it goes in a launch of its own
   if (tc_ok) {
     size_t keep = 0;
     for (size_t i = 0; i < seg->groups.size(); ++i) {
-      if (seg->groups[i].row_count > most_small && (seg->group_line[i] >= 0 || tc_shared_ok)) {
-        big.groups.push_back(seg->groups[i]);
-        big.group_line.push_back(seg->group_line[i]);
+      const bool shared = seg->group_line[i] < 0;
+      const bool many = w.quant4 && !shared ? q4_tc : seg->groups[i].row_count > kSplitChunkedMaxRows;
+      if (many && (!shared || tc_shared_ok)) {
+        Segment& to = shared && w.quant4 ? big_shared : big;
+        to.groups.push_back(seg->groups[i]);
+        to.group_line.push_back(seg->group_line[i]);
       } else {
         seg->groups[keep] = seg->groups[i];
         seg->group_line[keep] = seg->group_line[i];
@@ -668,70 +710,29 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
     }
     seg->groups.resize(keep);
     seg->group_line.resize(keep);
-    if (w.quant4 && !big.groups.empty() && !q4_scratch_ready(c, w, (int)big.groups.size())) {
-      seg->groups.insert(seg->groups.end(), big.groups.begin(), big.groups.end());
-      seg->group_line.insert(seg->group_line.end(), big.group_line.begin(), big.group_line.end());
-      big.groups.clear();
-      big.group_line.clear();
+  }
+  for (Segment* part : {&big, &big_shared})
+    if (!part->groups.empty()) {
+      int rc = flush_segment_tc(c, part, w, x, n_rows, s, w.quant4 && part == &big);
+      if (rc != PM_OK) return rc;
+    }
+  if (w.quant4) {  // the shared expert of a uint4 layer is bf16
+    std::vector<pm_ffn_group> shared;
+    size_t keep = 0;
+    for (size_t i = 0; i < seg->groups.size(); ++i) {
+      if (seg->group_line[i] < 0) shared.push_back(seg->groups[i]);
+      else seg->groups[keep++] = seg->groups[i];
+    }
+    seg->groups.resize(keep);
+    if (!shared.empty()) {
+      int rc = flush_groups_split(c, shared, false, true, w, x, desc_used, s);
+      if (rc != PM_OK) return rc;
     }
   }
-  if (!big.groups.empty()) {
-    int rc = flush_segment_tc(c, &big, w, x, n_rows, s, w.quant4 != 0);
+  if (!seg->groups.empty()) {
+    int rc = flush_groups_split(c, seg->groups, w.quant4 != 0, tc_ok, w, x, desc_used, s);
     if (rc != PM_OK) return rc;
   }
-  if (seg->groups.empty()) {
-    if (!seg->lines.empty()) {
-      cudaEvent_t ev = next_seg_event(c);
-      PM_CUDA(cudaEventRecord(ev, s));
-      for (int line : seg->lines) c->line_read[line] = ev;
-    }
-    seg->lines.clear();
-    seg->waits.clear();
-    return PM_OK;
-  }
-  FfnPlanInfo info;
-  // without the tensor-core path (shapes it cannot tile) larger groups stay in 64-row chunks for the staged kernel
-  const int chunk_rows = (w.quant4 || tc_ok) ? kSplitMaxRows : kMaxChunkRows;
-  int rc = plan_groups_size(seg->groups.data(), (int)seg->groups.size(), w.hidden, &info, chunk_rows);
-  if (rc != PM_OK) return rc;
-  if (*desc_used + info.blob_bytes() > c->plan_cap) return fail(PM_ERR_STATE, "launch plan buffer overflow");
-  Stage st = stage_of(c);
-  rc = plan_groups_into(seg->groups.data(), (int)seg->groups.size(), w.hidden, st.plan + *desc_used,
-                        c->plan_cap - *desc_used, &info, chunk_rows);
-  if (rc != PM_OK) return rc;
-  PM_CUDA(cudaMemcpyAsync(c->d_plan + *desc_used, st.plan + *desc_used, info.blob_bytes(), cudaMemcpyHostToDevice, s));
-  pm_ctx::FfnSample sample{};
-  if (c->profile_ffn) {
-    auto take_event = [&](cudaEvent_t* e) -> cudaError_t {
-      if (!c->ffn_event_pool.empty()) {
-        *e = c->ffn_event_pool.back();
-        c->ffn_event_pool.pop_back();
-        return cudaSuccess;
-      }
-      return cudaEventCreate(e);
-    };
-    sample.fused = ffn_launch_is_fused(info, w.quant4);
-    PM_CUDA(take_event(&sample.e0));
-    if (!sample.fused) PM_CUDA(take_event(&sample.e1));
-    PM_CUDA(take_event(&sample.e2));
-    for (const pm_ffn_group& g : seg->groups) {
-      int64_t mat = (int64_t)g.inter * w.hidden;
-      // uint4: half a byte per weight plus one fp16 {scale, zero} pair per 128 weights
-      int64_t one = w.quant4 ? mat / 2 + mat / 128 * 4 : mat * 2;
-      sample.bytes_gu += 2 * one;
-      sample.bytes_dn += one;
-    }
-    PM_CUDA(cudaEventRecord(sample.e0, s));
-  }
-  PM_CUDA(launch_swiglu_ffn(c->d_plan + *desc_used, info, w.quant4, x, w.hidden, c->d_row_token, c->d_hbuf,
-                            c->ws_inter, c->d_yexp, s, (c->profile_ffn && !sample.fused) ? sample.e1 : nullptr,
-                            c->d_tc_err));
-  if (c->profile_ffn) {
-    PM_CUDA(cudaEventRecord(sample.e2, s));
-    c->ffn_samples.push_back(sample);
-  }
-  c->kernel_launches += ffn_launch_is_fused(info, w.quant4) ? 1 : 2;
-  *desc_used += align_up(info.blob_bytes(), 256);
   if (!seg->lines.empty()) {
     cudaEvent_t ev = next_seg_event(c);
     PM_CUDA(cudaEventRecord(ev, s));
@@ -741,7 +742,6 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
   seg->group_line.clear();
   seg->lines.clear();
   seg->waits.clear();
-  (void)n_rows;
   return PM_OK;
 }
 
@@ -1016,7 +1016,6 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   c->tc_plan_used = 0;
   c->xperm_ready = false;
   c->tc_maps_ready = false;
-  c->tc_maps_q4_ready = false;
   if (c->profile_ffn && !c->ffn_samples.empty()) {  // their events have fired: recycle them now
     rc = rt_profile_collect(c);
     if (rc != PM_OK) return rc;
@@ -1278,7 +1277,6 @@ pm_ctx::~pm_ctx() {
   if (ws_dev) cudaFree(ws_dev);
   if (h_stage) cudaFreeHost(h_stage);
   if (h_tc_plan) cudaFreeHost(h_tc_plan);
-  if (q4_scratch) cudaFree(q4_scratch);
   if (d_topn) cudaFree(d_topn);
   if (h_topn) cudaFreeHost(h_topn);
   if (h_routed_scores) cudaFreeHost(h_routed_scores);

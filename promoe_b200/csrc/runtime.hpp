@@ -151,13 +151,7 @@ struct pm_ctx {
   int32_t* d_topn = nullptr;
   int32_t* h_topn = nullptr;
   int64_t topn_launches = 0;
-  // uint4 experts on the prefill path: the packed weights of a segment's experts are expanded into
-  // this bf16 slab (one line per expert of the segment) and the tensor-core kernels read it
-  unsigned char* q4_scratch = nullptr;
-  size_t q4_scratch_lines = 0, q4_scratch_stride = 0;
-  pm::TcMaps tc_maps_q4;
-  bool tc_maps_q4_ready = false;  // per layer call
-  int64_t q4_expanded = 0;        // experts expanded so far
+  int64_t q4_expanded = 0;        // uint4 experts that ran on the tensor cores so far (expanded to bf16 on the way)
 
   bool keep_routing = false;
   int seq_len = 1;
@@ -236,8 +230,6 @@ bool tc_prefill_usable(const pm_ctx* c, const pm_layer_weights& w);
 bool tc_prefill_usable_q4(const pm_ctx* c, const pm_layer_weights& w);
 bool tc_shared_usable(const pm_layer_weights& w);  // one tensor map can span the shared gate and up matrices
 int tc_build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m);
-// Same with the routed experts' bf16 weights in `slab` (gate, up, down back to back in every line).
-int tc_build_maps_q4(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m);
 void tc_tile_count(const TcGroup& g, int hidden, int* gu, int* dn);  // adds the group's tiles
 
 }  // namespace pm

@@ -11,6 +11,21 @@ namespace sm100 {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// Shared memory by 32-bit address (pointers that went through integer arithmetic would become generic).
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
@@ -25,17 +40,16 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 
 // Waits for the barrier's phase `parity`, for about two seconds at most. Returns false on give-up, or as
 // soon as *abort (a flag in shared memory that another role of the block sets when it gives up) is seen.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile int* abort) {
-  const uint32_t addr = smem_u32(bar);
+__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity, const volatile int* abort) {
   long long t0 = 0;
   for (uint32_t i = 0;; ++i) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done)
-        : "r"(addr), "r"(parity)
+        : "r"(addr), "r"(parity), "r"(100000u)  // the thread may sleep this many ns per poll
         : "memory");
     if (done) return true;
     if ((i & 15) == 15) {
@@ -45,6 +59,24 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
       if (t - t0 > 4000000000ll) return false;
     }
   }
+}
+
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile int* abort) {
+  return mbar_wait(smem_u32(bar), parity, abort);
+}
+
+// Both barriers, their first polls under way together (a poll takes some 150 cycles even when it succeeds).
+__device__ __forceinline__ bool mbar_wait2(uint32_t a, uint32_t parity_a, uint32_t b, uint32_t parity_b, const volatile int* abort) {
+  uint32_t da, db;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%2], %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 q, [%4], %5;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\tselp.u32 %1, 1, 0, q;\n\t}"
+      : "=r"(da), "=r"(db)
+      : "r"(a), "r"(parity_a), "r"(b), "r"(parity_b)
+      : "memory");
+  return (da || mbar_wait(a, parity_a, abort)) && (db || mbar_wait(b, parity_b, abort));
 }
 
 // ---- CTA pairs (clusters of two) ----------------------------------------------------------------
@@ -62,8 +94,14 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ void mbar_arrive(uint32_t addr) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// Arrival on a barrier of either CTA of the pair. What it announces is this CTA's own shared or tensor memory,
+// ordered for the tensor core by fence.proxy.async / tcgen05 fences before the call, so CTA scope does:
+// cluster scope would wait for every outstanding write of the thread (1 us and more per call).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // TMA: global (tensor map) -> this CTA's shared memory, completion counted in bytes on `bar`, a cluster
@@ -90,6 +128,14 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, u
 }
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+
+// 4 bytes global -> shared without registers; the calling thread's copies so far arrive on `bar` when done.
+__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // ---- tensor memory ----------------------------------------------------------------------------

@@ -42,12 +42,6 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   return r;
 }
 
-__device__ __forceinline__ uint32_t ldg_stream_u32(const uint32_t* p) {
-  uint32_t r;
-  asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(r) : "l"(p));
-  return r;
-}
-
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
                                          uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
@@ -1003,31 +997,6 @@ cudaError_t dispatch_nt(int max_rows, const GroupDesc* groups, const int32_t* ti
   return launch_one<8, NMAT>(groups, tile_group, tiles, bsrc, ldb, row_token, hidden, maxK, hbuf, ld_h, yexp, s);
 }
 
-// Expands one uint4 group-128 matrix [rows, K] into bf16 (for the prefill path, which reads bf16 tiles
-// by TMA): a thread turns one 32-bit word (8 weights: even-k nibbles in the low half, odd-k nibbles in
-// the high half) into 16 bytes of bf16, w = (q - zero) * scale in float32, rounded once.
-__global__ void __launch_bounds__(256)
-dequant_q4_kernel(const uint32_t* __restrict__ packed, const uint32_t* __restrict__ sz, size_t n_words,
-                  int words_per_row, uint4* __restrict__ out) {
-  const int groups_per_row = words_per_row / 16;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_words; i += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t w = ldg_stream_u32(packed + i);
-    const size_t row = i / words_per_row;
-    const int wc = (int)(i - row * words_per_row);
-    const uint32_t m = __ldg(sz + row * groups_per_row + wc / 16);
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&m));  // x = scale, y = zero
-    uint32_t o[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float even = ((float)((w >> (4 * j)) & 0xFu) - f.y) * f.x;
-      const float odd = ((float)((w >> (16 + 4 * j)) & 0xFu) - f.y) * f.x;
-      const __nv_bfloat162 pair = __floats2bfloat162_rn(even, odd);
-      o[j] = *reinterpret_cast<const uint32_t*>(&pair);
-    }
-    out[i] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
-}
-
 }  // namespace
 
 cudaError_t launch_resident_ffn(const ResidentArgs& r, int32_t* counters, int32_t* err, int max_rows,
@@ -1106,16 +1075,6 @@ cudaError_t launch_swiglu_ffn(const unsigned char* blob_dev, const FfnPlanInfo& 
   }
   return dispatch_nt<1>(max_rows, groups, t_dn, info.tiles_dn, hbuf, ld_h, row_token, H, ld_h, nullptr, ld_h,
                         yexp, s);
-}
-
-cudaError_t launch_dequant_q4(const void* packed, const void* scale_zero, int rows, int K, __nv_bfloat16* out,
-                              cudaStream_t s) {
-  if (rows <= 0 || K <= 0 || K % 128 != 0) return cudaErrorInvalidValue;
-  const size_t n_words = (size_t)rows * (K / 8);
-  const unsigned blocks = (unsigned)std::min<size_t>((n_words + 255) / 256, 148 * 16);
-  dequant_q4_kernel<<<blocks, 256, 0, s>>>((const uint32_t*)packed, (const uint32_t*)scale_zero, n_words, K / 8,
-                                           (uint4*)out);
-  return cudaGetLastError();
 }
 
 }  // namespace pm

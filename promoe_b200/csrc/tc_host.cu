@@ -25,14 +25,17 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// bf16 tensor, innermost dimension k, 64 k (128 bytes) wide boxes, 128-byte swizzle, zero fill.
+// Innermost dimension k, zero fill. bf16: boxes 64 k (128 bytes) wide, 128-byte swizzle. Packed uint4
+// (as bytes): boxes 128 k (64 bytes) wide, 64-byte swizzle, so that threads reading 16 bytes of
+// neighbouring rows meet different banks.
 int encode(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides_bytes,
-           const cuuint32_t* box) {
+           const cuuint32_t* box, bool packed = false) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return fail(PM_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
   cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims, strides_bytes,
-                  box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+  CUresult r = fn(map, packed ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank,
+                  const_cast<void*>(base), dims, strides_bytes, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  packed ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(PM_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult " + std::to_string((int)r));
   return PM_OK;
@@ -52,21 +55,23 @@ int encode_rows(CUtensorMap (&maps)[4], const void* base, uint64_t k, uint64_t r
 
 // Gate and up projections [inter, hidden] of `lines` experts `stride` bytes apart, as one map.
 int encode_gate_up(CUtensorMap* map, int32_t* up_first, const unsigned char* gate, const unsigned char* up, uint64_t hidden,
-                   uint64_t inter, uint64_t stride, uint64_t lines) {
+                   uint64_t inter, uint64_t stride, uint64_t lines, bool packed = false) {
   *up_first = up < gate;
   const unsigned char* base = std::min(gate, up);
   const uint64_t apart = (uint64_t)(std::max(gate, up) - base);
-  cuuint64_t dims[5] = {hidden, 16, 2, inter / 16, lines};
-  cuuint64_t strides[4] = {hidden * 2, apart, hidden * 32, stride};
+  const uint64_t pitch = packed ? hidden / 2 : hidden * 2;
+  cuuint64_t dims[5] = {packed ? hidden / 2 : hidden, 16, 2, inter / 16, lines};
+  cuuint64_t strides[4] = {pitch, apart, pitch * 16, stride};
   cuuint32_t box[5] = {64, 16, 2, 4, 1};
-  return encode(map, base, 5, dims, strides, box);
+  return encode(map, base, 5, dims, strides, box, packed);
 }
 
-int encode_down(CUtensorMap* map, const void* down, uint64_t hidden, uint64_t inter, uint64_t stride, uint64_t lines) {
-  cuuint64_t dims[3] = {inter, hidden, lines};
-  cuuint64_t strides[2] = {inter * 2, stride};
+int encode_down(CUtensorMap* map, const void* down, uint64_t hidden, uint64_t inter, uint64_t stride, uint64_t lines,
+                bool packed = false) {
+  cuuint64_t dims[3] = {packed ? inter / 2 : inter, hidden, lines};
+  cuuint64_t strides[2] = {packed ? inter / 2 : inter * 2, stride};
   cuuint32_t box[3] = {64, 128, 1};
-  return encode(map, down, 3, dims, strides, box);
+  return encode(map, down, 3, dims, strides, box, packed);
 }
 
 }  // namespace
@@ -89,20 +94,19 @@ bool tc_shared_usable(const pm_layer_weights& w) {
   return (g > u ? g - u : u - g) < ((uintptr_t)1 << 40);
 }
 
-namespace {
-
-// Maps of the token rows, of a slab of bf16 expert lines (`lines` lines `stride` bytes apart, the
-// three matrices at the given addresses of line 0) and of the layer's shared expert.
-int build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, const unsigned char* gate0,
-               const unsigned char* up0, const unsigned char* down0, uint64_t stride, uint64_t lines, TcMaps* m) {
-  const uint64_t H = w.hidden, I = w.inter, Is = w.shared_inter;
+// Maps of the token rows, of the slab of expert lines and of the layer's shared expert. uint4 layers: the
+// slab maps describe the packed matrices.
+int tc_build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m) {
+  const uint64_t H = w.hidden, I = w.inter, Is = w.shared_inter, stride = c->line_stride, lines = c->n_lines;
+  const bool packed = w.quant4 != 0;
   int rc = encode_rows(m->a_x, c->d_xperm, H, (uint64_t)rows_cap, H);
   if (rc != PM_OK) return rc;
   rc = encode_rows(m->a_h, c->d_hbuf, (uint64_t)c->ws_inter, (uint64_t)rows_cap, (uint64_t)c->ws_inter);
   if (rc != PM_OK) return rc;
-  rc = encode_gate_up(&m->slab_gu, &m->slab_up_first, gate0, up0, H, I, stride, lines);
+  rc = encode_gate_up(&m->slab_gu, &m->slab_up_first, c->slab + c->param_offset[c->role_gate],
+                      c->slab + c->param_offset[c->role_up], H, I, stride, lines, packed);
   if (rc != PM_OK) return rc;
-  rc = encode_down(&m->slab_down, down0, H, I, stride, lines);
+  rc = encode_down(&m->slab_down, c->slab + c->param_offset[c->role_down], H, I, stride, lines, packed);
   if (rc != PM_OK) return rc;
   if (Is > 0 && tc_shared_usable(w)) {  // one "line"; its stride is never used but has to be a valid one
     rc = encode_gate_up(&m->sh_gu, &m->sh_up_first, (const unsigned char*)w.shared_w_gate, (const unsigned char*)w.shared_w_up, H,
@@ -116,19 +120,6 @@ int build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, const unsigne
     m->sh_up_first = 0;
   }
   return PM_OK;
-}
-
-}  // namespace
-
-int tc_build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m) {
-  return build_maps(c, w, rows_cap, c->slab + c->param_offset[c->role_gate], c->slab + c->param_offset[c->role_up],
-                    c->slab + c->param_offset[c->role_down], (uint64_t)c->line_stride, (uint64_t)c->n_lines, m);
-}
-
-int tc_build_maps_q4(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m) {
-  const size_t mat = (size_t)w.inter * w.hidden * 2;
-  return build_maps(c, w, rows_cap, c->q4_scratch, c->q4_scratch + mat, c->q4_scratch + 2 * mat,
-                    (uint64_t)c->q4_scratch_stride, (uint64_t)c->q4_scratch_lines, m);
 }
 
 // Tiles of one group: token tiles of at most kTcMaxN rows times blocks of 128 gate/up rows or 256 down rows.

@@ -7,9 +7,11 @@ import pytest
 import torch
 
 from oracle import moe_math as om
+from oracle import quant4 as oq
 from promoe_b200 import _lib
+from promoe_b200 import quant4 as pq
 from promoe_b200.engine import ExpertCache
-from tests.helpers import TinyModel, dev_bf16
+from tests.helpers import TinyModel, bf16_weights, dev_bf16
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +68,73 @@ def test_tile_edges(lib, H, I, counts):
 
 def test_up_matrix_first_in_memory(lib):
     assert run_routed(lib, 256, 192, [70, 130, 33], names=("up_proj.weight", "down_proj.weight", "gate_proj.weight")) > 0
+
+
+@pytest.mark.parametrize("H,I,counts", [
+    (128, 128, [64, 0, 70]),              # one k-step
+    (640, 384, [129, 256, 257, 3]),       # either side of a full token tile, ragged weight tiles
+    (1024, 1152, [600, 64]),              # K loops longer than the rings, two and three token tiles
+    (256, 256, [65] * 24),                # more tiles than CTA pairs
+])
+def test_uint4_tile_edges(lib, H, I, counts):
+    rng = np.random.default_rng(H + I)
+    E, deq = len(counts), []
+    cache = ExpertCache(1, E, num_expert_per_token=1, cache_rate=1.0, num_predict_expert_per_layer=0)
+    cache.set_param_list(["w1.qweight", "w1.scale_zero", "w3.qweight", "w3.scale_zero", "w2.qweight", "w2.scale_zero"])
+    for e in range(E):
+        raw, mats = [], []
+        for shape in ((I, H), (I, H), (H, I)):
+            packed, sz = pq.quantize_pack(bf16_weights(rng, shape))
+            raw += [packed, sz]
+            mats.append(oq.dequantize(packed, sz))
+        deq.append(mats)
+        cache.register_expert(0, e, raw)
+    cache.pin_all()
+    cache.build_slab()
+    cache.set_layer_weights(0, None, I, 1, False, 1.0, hidden=H, quant4=True)
+    ids = np.repeat(np.arange(E, dtype=np.int32), counts)
+    rng.shuffle(ids)
+    n = len(ids)
+    x = om.bf16_round(rng.standard_normal((n, H)).astype(np.float32))
+    xd, idd = dev_bf16(x), torch.from_numpy(ids).cuda()
+    out = torch.full((n, H), float("nan"), dtype=torch.float32, device="cuda")
+    for _ in range(2):
+        _lib.call("pm_moe_forward_routed", cache.handle, 0, xd.data_ptr(), n, idd.data_ptr(), out.data_ptr(), 0, None, None,
+                  0, 0, 0, 0, None)
+        torch.cuda.synchronize()
+    assert cache.get("tc_error") == "0" and int(cache.get("q4_expanded")) > 0
+    cache.close()
+    got, ref = out.cpu().numpy(), np.zeros((n, H))
+    for e in range(E):
+        if counts[e]:
+            ref[ids == e] = om.swiglu_mlp(x[ids == e], *deq[e], round_h_bf16=True)
+    # weights rounded to bf16 after dequantisation: 2^-9 per product, independent, on top of the bf16 path's error
+    np.testing.assert_allclose(got, ref, rtol=3e-2, atol=3e-2 * np.abs(ref).max() * 0.25)
+    assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 8e-3
+
+
+def test_uint4_layer_with_bf16_shared_expert(lib):
+    """The shared expert of a uint4 layer is bf16: decode rows and prompt rows both reach it."""
+    model = TinyModel(seed=8, L=1, E=4, H=256, I=128, k=2, shared_I=192)
+    rng = np.random.default_rng(3)
+    cache = ExpertCache(1, 4, num_expert_per_token=2, cache_rate=1.0, num_predict_expert_per_layer=0)
+    cache.set_param_list(["w1.qweight", "w1.scale_zero", "w3.qweight", "w3.scale_zero", "w2.qweight", "w2.scale_zero"])
+    for e in range(4):
+        raw, mats = [], []
+        for w in model.experts[0][e]:
+            packed, sz = pq.quantize_pack(w)
+            raw += [packed, sz]
+            mats.append(oq.dequantize(packed, sz))
+        model.experts[0][e] = tuple(mats)
+        cache.register_expert(0, e, raw)
+    cache.pin_all()
+    cache.build_slab()
+    cache.set_layer_weights(0, dev_bf16(model.gate_w[0]), model.I, 2, False,
+                            gate_bias=None if model.gate_bias is None else torch.from_numpy(model.gate_bias[0]).cuda(),
+                            shared=[dev_bf16(w) for w in model.shared[0]], quant4=True)
+    for T in (5, 40, 300):
+        x = om.bf16_round(rng.standard_normal((T, model.H)).astype(np.float32))
+        y = cache.forward(0, dev_bf16(x)).float().cpu().numpy()
+        ref, _, _ = model.oracle_forward(0, x)
+        assert np.linalg.norm(y - ref) / np.linalg.norm(ref) < 8e-3
+    cache.close()
