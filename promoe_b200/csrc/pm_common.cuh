@@ -51,11 +51,13 @@ constexpr int kMaxChunkRows = 64;   // token rows per chunk (8 MMA n-tiles)
 constexpr int kSplitMaxRows = 16;   // launches whose chunks all fit use the split-K decode kernel,
 constexpr int kSplitTileGu = 16;    // whose tiles are 16 gate+up rows
 constexpr int kSplitTileDn = 32;    // or 32 down rows
-// Most rows of a bf16 group that still runs as 16-row chunks of the split-K kernel; above, one tensor-core
-// tile streams its weights once. Measured on a layer of 64 tokens x top-8 over experts of 1-40 rows
-// (hidden 3584, inter 2560, shared 20480): FFN 796 us with this line at 32, 874 us at 64; a prompt of 777
-// tokens x top-4 over 60 experts: 326 us at 32, 382 us at 64. (At 16 a decode batch of 32 loses 45 us: its
-// shared expert alone then costs a launch pair of its own.)
+// Most rows of a bf16 group for which its segment stays on the split-K kernel (as chunks of 16 rows). One group
+// above it takes all groups of the segment to the tensor cores, whose launch pair streams the weights of
+// every group once; two kinds of launches after one another each leave SMs idle at their ends. Measured
+// (FFN of one layer, mixed launches with the same line -> one kind): 64 tokens x top-8, experts of 1-40 rows
+// (hidden 3584, inter 2560, shared 20480) 773 -> 716 us; 100 / 200 / 400 / 777 tokens x top-4 over 60 experts
+// (2048 x 1408, shared 5632) 224 -> 204, 254 -> 228, 279 -> 247, 314 -> 269 us. With the line at 0, 32 tokens x
+// top-6 over 64 experts lose: 155 us in chunks against 177 us.
 constexpr int kSplitChunkedMaxRows = 32;
 
 // Kernel launchers (defined in the .cu files). All take the caller's stream.

@@ -685,19 +685,20 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
       c->line_waiter[line] = s;
     }
   }
-  // Groups with many rows go to the tensor cores; the others stay on the split-K tiles, which stream
-  // the weights faster when there are only a few rows to use them for (a large decode batch has both
-  // kinds in one layer call). Below the line a group runs as chunks of 16 rows through the split-K
-  // tiles: its weights are read once from HBM and again from L2 for the later chunks.
+  // A segment with groups of many rows goes to the tensor cores; otherwise the split-K tiles stream the
+  // weights faster when there are only a few rows to use them for. There a group runs as chunks of 16 rows:
+  // its weights are read once from HBM and again from L2 for the later chunks.
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
   const bool tc_shared_ok = tc_shared_usable(w);
   const bool q4_tc = w.quant4 && tc_ok && q4_prefers_tc(*seg);
+  bool bf16_tc = false;
+  for (const pm_ffn_group& g : seg->groups) bf16_tc = bf16_tc || g.row_count > kSplitChunkedMaxRows;
   Segment big, big_shared;  // the shared expert of a uint4 layer is bf16: it goes in a launch of its own
   if (tc_ok) {
     size_t keep = 0;
     for (size_t i = 0; i < seg->groups.size(); ++i) {
       const bool shared = seg->group_line[i] < 0;
-      const bool many = w.quant4 && !shared ? q4_tc : seg->groups[i].row_count > kSplitChunkedMaxRows;
+      const bool many = !w.quant4 ? bf16_tc : shared ? seg->groups[i].row_count > kSplitChunkedMaxRows : q4_tc;
       if (many && (!shared || tc_shared_ok)) {
         Segment& to = shared && w.quant4 ? big_shared : big;
         to.groups.push_back(seg->groups[i]);
