@@ -67,6 +67,26 @@ cudaError_t launch_gate_topk(const __nv_bfloat16* x, const __nv_bfloat16* w_gate
                              int32_t* topk_ids, float* topk_w, int32_t* topk_slot,
                              float* shared_scale, float* logits_out, cudaStream_t s);
 
+// Router and permutation of a decode batch (at most 16 tokens) in one launch: launch_gate_topk followed by
+// launch_permute on its ids. Usable when the token rows fit shared memory.
+struct RouteArgs {
+  const __nv_bfloat16 *x, *w_gate;
+  const float* bias;
+  const __nv_bfloat16* w_shared_gate;
+  int32_t T, H, E, k, norm_topk;
+  float routed_scale;
+  const int32_t* expert_slot;
+  int32_t* topk_ids;
+  float* topk_w;
+  int32_t* topk_slot;
+  float* shared_scale;
+  int32_t *counts, *offsets, *row_token, *pos, *err_flag;
+  int32_t tail_rows, zero_n;
+  int32_t* zero_words;
+};
+bool route_small_usable(int T, int H);
+cudaError_t launch_route_small(const RouteArgs& a, cudaStream_t s);
+
 // zero_words / zero_n: an int32 array the permutation also clears (the dependency counters of the
 // fused FFN launch that follows on the same stream), or nullptr.
 cudaError_t launch_permute(const int32_t* topk_ids, int R, int k, int E, int32_t* counts,

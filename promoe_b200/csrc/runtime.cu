@@ -156,7 +156,7 @@ int ensure_workspace(pm_ctx* c, int T, const pm_layer_weights& w) {
   // the groups of every expert and the shared one, and a 256-byte rounding per segment (at most one per expert)
   c->tc_plan_cap = (sizeof(TcGroup) + 256) * ((size_t)E + 2);
   size_t o_tcp = take(c->tc_plan_cap);
-  c->perm_scratch_ints = (R / 4096 + 2) * (size_t)E;
+  c->perm_scratch_ints = (R / 1024 + 2) * (size_t)E;
   size_t o_ps = take(c->perm_scratch_ints * 4);
   PM_CUDA(cudaMalloc(&c->ws_dev, off));
   PM_CUDA(cudaMemset(c->ws_dev, 0, off));
@@ -874,22 +874,36 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
     PM_CUDA(cudaMemcpyAsync(ly.slot_table_dev, st.slot_table, (size_t)E * 4, cudaMemcpyHostToDevice, s));
     ly.slot_table_dirty = false;
   }
-  const int32_t* ids_dev = c->d_topk_ids;
-  if (routed) {
-    ids_dev = routed->row_expert;
-  } else {
-    PM_CUDA(launch_gate_topk(x, (const __nv_bfloat16*)w.gate_w, w.gate_bias, (const __nv_bfloat16*)w.shared_gate_w,
-                             T, H, E, k, w.norm_topk, w.routed_scale, ly.slot_table_dev, c->d_topk_ids,
-                             c->d_topk_w, c->d_topk_slot, c->d_shared_scale, nullptr, s));
-    c->kernel_launches += 1;
-  }
   // rows per expert <= T, or the bound the caller of the routed-rows form guarantees
   const int row_bound = (routed && routed->max_rows_per_expert > 0) ? std::min(T, routed->max_rows_per_expert) : T;
   const bool spec = c->device_plan && !w.quant4 && resident_ffn_available(row_bound);
-  PM_CUDA(launch_permute(ids_dev, R, k, E, c->d_counts, c->d_offsets, c->d_row_token, c->d_pos, c->d_err,
-                         n_shared * T, T, s, c->d_perm_scratch, c->perm_scratch_ints,
-                         spec ? c->d_res_counters : nullptr, kMaxFusedGroups + 1));
-  c->kernel_launches += 1;
+  int32_t* zero_words = spec ? c->d_res_counters : nullptr;
+  if (!routed && route_small_usable(T, H)) {
+    RouteArgs a{};
+    a.x = x; a.w_gate = (const __nv_bfloat16*)w.gate_w; a.bias = w.gate_bias;
+    a.w_shared_gate = (const __nv_bfloat16*)w.shared_gate_w;
+    a.T = T; a.H = H; a.E = E; a.k = k; a.norm_topk = w.norm_topk; a.routed_scale = w.routed_scale;
+    a.expert_slot = ly.slot_table_dev;
+    a.topk_ids = c->d_topk_ids; a.topk_w = c->d_topk_w; a.topk_slot = c->d_topk_slot; a.shared_scale = c->d_shared_scale;
+    a.counts = c->d_counts; a.offsets = c->d_offsets; a.row_token = c->d_row_token; a.pos = c->d_pos; a.err_flag = c->d_err;
+    a.tail_rows = n_shared * T;
+    a.zero_words = zero_words; a.zero_n = spec ? kMaxFusedGroups + 1 : 0;
+    PM_CUDA(launch_route_small(a, s));
+    c->kernel_launches += 1;
+  } else {
+    const int32_t* ids_dev = c->d_topk_ids;
+    if (routed) {
+      ids_dev = routed->row_expert;
+    } else {
+      PM_CUDA(launch_gate_topk(x, (const __nv_bfloat16*)w.gate_w, w.gate_bias, (const __nv_bfloat16*)w.shared_gate_w,
+                               T, H, E, k, w.norm_topk, w.routed_scale, ly.slot_table_dev, c->d_topk_ids,
+                               c->d_topk_w, c->d_topk_slot, c->d_shared_scale, nullptr, s));
+      c->kernel_launches += 1;
+    }
+    PM_CUDA(launch_permute(ids_dev, R, k, E, c->d_counts, c->d_offsets, c->d_row_token, c->d_pos, c->d_err,
+                           n_shared * T, T, s, c->d_perm_scratch, c->perm_scratch_ints, zero_words, kMaxFusedGroups + 1));
+    c->kernel_launches += 1;
+  }
   std::vector<int> pred_dsts;
   if (!routed && c->cfg.predict_from_moe_input && c->seq_len == 1) {
     rc = launch_predictors(c, layer, x, T, H, s, &pred_dsts);

@@ -35,7 +35,11 @@ def run_gate(lib, x, wg, bias, k, norm, scale=1.0, shared_gate=None, slots=None)
 
 @pytest.mark.parametrize("T,H,E,k,norm", [(1, 64, 4, 2, True), (8, 2048, 60, 4, False),
                                           (32, 2048, 64, 6, False), (16, 4096, 8, 2, True),
-                                          (64, 3584, 64, 8, False), (5, 2048, 256, 8, True)])
+                                          (64, 3584, 64, 8, False), (5, 2048, 256, 8, True),
+                                          # a CTA per token, 4 and 8 tokens per CTA (with a ragged last one),
+                                          # one and four expert rows per warp, a ragged last group of rows
+                                          (296, 72, 61, 4, False), (299, 512, 61, 4, False), (301, 4096, 8, 2, True),
+                                          (1779, 256, 66, 6, False), (1781, 264, 16, 2, False)])
 def test_gate_topk_bit_exact(lib, T, H, E, k, norm):
     rng = np.random.default_rng(1000 + T + E)
     x = om.bf16_round(rng.standard_normal((T, H)).astype(np.float32))
@@ -99,7 +103,9 @@ def run_permute(lib, ids, E):
 
 
 @pytest.mark.parametrize("T,k,E", [(1, 2, 8), (8, 4, 60), (32, 6, 64), (64, 8, 64), (512, 2, 8),
-                                   (2048, 6, 64), (3, 8, 256)])
+                                   (2048, 6, 64), (3, 8, 256),
+                                   # one, exactly one, just over one and several rounds of 1024 pairs
+                                   (256, 4, 60), (1025, 1, 256), (777, 4, 60), (5000, 2, 5)])
 def test_permute_bit_exact(lib, T, k, E):
     rng = np.random.default_rng(7 + T)
     ids = np.stack([rng.choice(E, size=k, replace=False) for _ in range(T)]).astype(np.int32)

@@ -228,3 +228,24 @@ def test_routed_rows_reject_an_expert_id_out_of_range(lib):
         ref = om.swiglu_mlp(x[r:r + 1], *model.experts[0][e_id], round_h_bf16=True)
         np.testing.assert_allclose(got[r:r + 1], ref, rtol=RTOL, atol=RTOL * np.abs(ref).max() * 0.25)
     cache.close()
+
+
+@pytest.mark.parametrize("T,E,k,H,shared", [(1, 7, 1, 64, True), (2, 64, 6, 320, False), (5, 60, 4, 2048, True),
+                                            (16, 256, 16, 128, True), (16, 9, 9, 192, False), (13, 63, 8, 576, True)])
+def test_decode_router_bit_exact(lib, T, E, k, H, shared):
+    """Batches of up to 16 tokens are routed and permuted by one cluster: ids, weights and the layer's output
+    (which needs the permutation) against the canonical order and the oracle, at ragged splits of the rows."""
+    model = TinyModel(seed=40 + T + E, L=1, E=E, H=H, I=64, k=k, shared_I=64 if shared else 0, shared_gate=shared)
+    cache = model.make_cache(cache_rate=1.0, num_predict_expert_per_layer=0)
+    cache.set("keep_routing", 1)
+    for x in model.hidden_stream(T, 2):
+        y = cache.forward(0, dev_bf16(x))
+        torch.cuda.synchronize()
+        ids, w = cache.last_routing(0, T, k)
+        ref_ids, ref_w = model.canonical_routing(0, x)
+        assert np.array_equal(ids, ref_ids.astype(np.int32))
+        np.testing.assert_allclose(w, ref_w, rtol=1e-4)
+        ref, _, _ = model.oracle_forward(0, x)
+        got = y.float().cpu().numpy()
+        np.testing.assert_allclose(got, ref, rtol=2e-2, atol=2e-2 * np.abs(ref).max() * 0.25)
+    cache.close()
