@@ -208,8 +208,13 @@ __device__ __forceinline__ uint4 load_b(const unsigned char* p) {
 // where both sums come out of the tensor core (the second from an all-ones A fragment).
 // Layout of the metadata: per matrix an array [rows, K/128] of {scale, zero} fp16 pairs.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t q4_pair(uint32_t word, int j) {
-  return ((word >> (4 * j)) & 0x000F000Fu) | 0x43004300u;
+// `ex` is kQ4Exponent in a register that the compiler cannot see through (a kernel argument): a logic instruction
+// takes one immediate, so with both constants known it spends two instructions instead of one.
+constexpr uint32_t kQ4Exponent = 0x43004300u;
+__device__ __forceinline__ uint32_t q4_pair(uint32_t word, int j, uint32_t ex) {
+  uint32_t r;
+  asm("lop3.b32 %0, %1, 0x000F000F, %2, 0xEA;" : "=r"(r) : "r"(word >> (4 * j)), "r"(ex));  // (a & mask) | ex
+  return r;
 }
 
 template <int NT, bool GATEUP, int DEPTH, bool COHERENT_B>
@@ -217,7 +222,7 @@ __device__ __forceinline__ void splitk_tile_q4(const GroupDesc& grp, int tile_lo
                                                const __nv_bfloat16* __restrict__ bsrc, int ldb,
                                                const int32_t* __restrict__ row_token, int hidden,
                                                __nv_bfloat16* __restrict__ hbuf, int ld_h,
-                                               float* __restrict__ yexp, float (*red)[2 * NT * 4][32]) {
+                                               float* __restrict__ yexp, float (*red)[2 * NT * 4][32], uint32_t ex) {
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int g = lane >> 2;
@@ -293,10 +298,10 @@ __device__ __forceinline__ void splitk_tile_q4(const GroupDesc& grp, int tile_lo
                                      : make_uint4(0, 0, 0, 0);
             const uint32_t w00 = (&a[d][0].x)[v], w01 = (&a[d][1].x)[v];  // matrix 0: rows g, g+8
             const uint32_t w10 = (&a[d][2].x)[v], w11 = (&a[d][3].x)[v];  // matrix 1
-            mma_bf16(raw[0], q4_pair(w00, 0), q4_pair(w01, 0), q4_pair(w00, 1), q4_pair(w01, 1), b.x, b.y);
-            mma_bf16(raw[0], q4_pair(w00, 2), q4_pair(w01, 2), q4_pair(w00, 3), q4_pair(w01, 3), b.z, b.w);
-            mma_bf16(raw[1], q4_pair(w10, 0), q4_pair(w11, 0), q4_pair(w10, 1), q4_pair(w11, 1), b.x, b.y);
-            mma_bf16(raw[1], q4_pair(w10, 2), q4_pair(w11, 2), q4_pair(w10, 3), q4_pair(w11, 3), b.z, b.w);
+            mma_bf16(raw[0], q4_pair(w00, 0, ex), q4_pair(w01, 0, ex), q4_pair(w00, 1, ex), q4_pair(w01, 1, ex), b.x, b.y);
+            mma_bf16(raw[0], q4_pair(w00, 2, ex), q4_pair(w01, 2, ex), q4_pair(w00, 3, ex), q4_pair(w01, 3, ex), b.z, b.w);
+            mma_bf16(raw[1], q4_pair(w10, 0, ex), q4_pair(w11, 0, ex), q4_pair(w10, 1, ex), q4_pair(w11, 1, ex), b.x, b.y);
+            mma_bf16(raw[1], q4_pair(w10, 2, ex), q4_pair(w11, 2, ex), q4_pair(w10, 3, ex), q4_pair(w11, 3, ex), b.z, b.w);
             mma_bf16(xs, kOnes, kOnes, kOnes, kOnes, b.x, b.y);
             mma_bf16(xs, kOnes, kOnes, kOnes, kOnes, b.z, b.w);
           }
@@ -350,12 +355,12 @@ __global__ void __launch_bounds__(kSplitThreads, 2)
 grouped_ffn_q4_kernel(const GroupDesc* __restrict__ groups, const int32_t* __restrict__ tile_group,
                       const __nv_bfloat16* __restrict__ bsrc, int ldb,
                       const int32_t* __restrict__ row_token, int hidden,
-                      __nv_bfloat16* __restrict__ hbuf, int ld_h, float* __restrict__ yexp) {
+                      __nv_bfloat16* __restrict__ hbuf, int ld_h, float* __restrict__ yexp, uint32_t ex) {
   constexpr bool GATEUP = (NMAT == 2);
   __shared__ float red[kSplitWarps][2 * NT * 4][32];
   const GroupDesc grp = groups[tile_group[blockIdx.x]];
   const int tile_local = blockIdx.x - (GATEUP ? grp.tile_start_gu : grp.tile_start_dn);
-  splitk_tile_q4<NT, GATEUP, DEPTH, false>(grp, tile_local, bsrc, ldb, row_token, hidden, hbuf, ld_h, yexp, red);
+  splitk_tile_q4<NT, GATEUP, DEPTH, false>(grp, tile_local, bsrc, ldb, row_token, hidden, hbuf, ld_h, yexp, red, ex);
 }
 
 template <int NT, int NMAT>
@@ -363,7 +368,7 @@ cudaError_t launch_q4(const GroupDesc* groups, const int32_t* tile_group, int ti
                       int ldb, const int32_t* row_token, int hidden, __nv_bfloat16* hbuf, int ld_h, float* yexp,
                       cudaStream_t s) {
   grouped_ffn_q4_kernel<NT, NMAT, 2><<<tiles, kSplitThreads, 0, s>>>(groups, tile_group, bsrc, ldb, row_token,
-                                                                     hidden, hbuf, ld_h, yexp);
+                                                                     hidden, hbuf, ld_h, yexp, kQ4Exponent);
   return cudaGetLastError();
 }
 
@@ -420,6 +425,7 @@ struct FusedLaunch {
   __nv_bfloat16* hbuf;
   float* yexp;
   int32_t hidden, ld_h;
+  uint32_t q4_exponent = kQ4Exponent;  // see q4_pair
 };
 
 // The split-K tile cut into stages, so that a resident CTA can have the first loads of its NEXT
@@ -556,7 +562,7 @@ __device__ __forceinline__ void tile_compute(const TileCtx<NT>& t, int s0, const
 // (see the layout note above q4_pair), then the per-group scale / zero fix-up.
 template <int NT, int DEPTH, bool COHERENT_B, int FIRST = 0, int COUNT = DEPTH>
 __device__ __forceinline__ void tile_compute_q4(const TileCtx<NT>& t, int s0, const uint4 (&a)[DEPTH][4],
-                                                const uint32_t (&sz)[DEPTH][4], float (&acc)[2][NT][4]) {
+                                                const uint32_t (&sz)[DEPTH][4], float (&acc)[2][NT][4], uint32_t ex) {
   constexpr uint32_t kOnes = 0x3F803F80u;  // bf16 (1, 1)
 #pragma unroll
   for (int d = FIRST; d < FIRST + COUNT; ++d) {
@@ -577,10 +583,10 @@ __device__ __forceinline__ void tile_compute_q4(const TileCtx<NT>& t, int s0, co
 #pragma unroll
         for (int h = 0; h < 2; ++h) {  // nibble pairs {0,1} go with b.x, b.y; pairs {2,3} with b.z, b.w
           // each word is unpacked once and used for every n-tile
-          const uint32_t a0 = q4_pair(w00, 2 * h), a1 = q4_pair(w01, 2 * h), a2 = q4_pair(w00, 2 * h + 1),
-                         a3 = q4_pair(w01, 2 * h + 1);
-          const uint32_t c0 = q4_pair(w10, 2 * h), c1 = q4_pair(w11, 2 * h), c2 = q4_pair(w10, 2 * h + 1),
-                         c3 = q4_pair(w11, 2 * h + 1);
+          const uint32_t a0 = q4_pair(w00, 2 * h, ex), a1 = q4_pair(w01, 2 * h, ex), a2 = q4_pair(w00, 2 * h + 1, ex),
+                         a3 = q4_pair(w01, 2 * h + 1, ex);
+          const uint32_t c0 = q4_pair(w10, 2 * h, ex), c1 = q4_pair(w11, 2 * h, ex), c2 = q4_pair(w10, 2 * h + 1, ex),
+                         c3 = q4_pair(w11, 2 * h + 1, ex);
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
             const uint32_t b0 = h ? bv[nt].z : bv[nt].x, b1 = h ? bv[nt].w : bv[nt].y;
@@ -731,7 +737,7 @@ __device__ __forceinline__ void stream_run(StreamState<NT, DEPTH>& st, const G* 
                                            const int32_t* __restrict__ row_token, int hidden,
                                            __nv_bfloat16* __restrict__ hbuf, int ld_h, float* __restrict__ yexp,
                                            float (*red2)[WARPS][2 * NT * 4][32], int32_t* counters, int32_t* total,
-                                           int total_target, int32_t* err) {
+                                           int total_target, int32_t* err, uint32_t ex) {
   constexpr bool COH = !GATEUP;  // the down phase reads rows other CTAs wrote in this kernel
   constexpr bool Q4 = std::is_same<G, FusedGroupQ4>::value;
   if (!st.active) return;
@@ -759,7 +765,7 @@ __device__ __forceinline__ void stream_run(StreamState<NT, DEPTH>& st, const G* 
     // with the steps DEPTH further on, so a warp always has loads outstanding while it waits.
     constexpr int HALF = DEPTH / 2;
     for (int s0 = 0; s0 < t.s_end; s0 += DEPTH) {
-      if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, 0, HALF>(t, s0, st.a, st.sz, acc);
+      if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, 0, HALF>(t, s0, st.a, st.sz, acc, ex);
       else tile_compute<NT, DEPTH, 0, HALF>(t, s0, st.a, st.b, acc);
       if (s0 + DEPTH < t.s_end) {
         tile_issue_a<NT, DEPTH, Q4, 0, HALF>(t, s0 + DEPTH, st.a, st.sz);
@@ -770,7 +776,7 @@ __device__ __forceinline__ void stream_run(StreamState<NT, DEPTH>& st, const G* 
         rows_loaded = true;
       }
       if (s0 + HALF < t.s_end) {
-        if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, HALF, HALF>(t, s0, st.a, st.sz, acc);
+        if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, HALF, HALF>(t, s0, st.a, st.sz, acc, ex);
         else tile_compute<NT, DEPTH, HALF, HALF>(t, s0, st.a, st.b, acc);
         if (s0 + DEPTH + HALF < t.s_end) {
           tile_issue_a<NT, DEPTH, Q4, HALF, HALF>(t, s0 + DEPTH, st.a, st.sz);
@@ -908,14 +914,14 @@ grouped_ffn_fused_kernel(const __grid_constant__ FusedLaunch a) {
   st.all_done = false;
   stream_begin<NT, true, DEPTH, WARPS>(st, sg, n, b, tiles_gu, a.x, a.hidden, a.row_token, a.hidden);
   stream_run<NT, true, DEPTH, WARPS>(st, sg, n, tiles_gu, a.x, a.hidden, a.row_token, a.hidden, a.hbuf, a.ld_h, a.yexp,
-                                     red, a.counters, a.total, total_target, a.err);
+                                     red, a.counters, a.total, total_target, a.err, a.q4_exponent);
   // This CTA's place in the one round-robin sequence continues into the down tiles, so the CTAs
   // that had one gate/up tile fewer take the first down tiles.
   const int n1 = b < tiles_gu ? (tiles_gu - b + grid - 1) / grid : 0;
   const int first_dn = b + n1 * grid - tiles_gu;
   stream_begin<NT, false, DEPTH, WARPS>(st, sg, n, first_dn, tiles_dn, a.hbuf, a.ld_h, a.row_token, a.hidden);
   stream_run<NT, false, DEPTH, WARPS>(st, sg, n, tiles_dn, a.hbuf, a.ld_h, a.row_token, a.hidden, nullptr, a.ld_h,
-                                      a.yexp, red, a.counters, a.total, total_target, a.err);
+                                      a.yexp, red, a.counters, a.total, total_target, a.err, a.q4_exponent);
 }
 
 // 8 warps x 2 CTAs per SM. (16 warps x 1 CTA, one batch of loads per tile, measured 28 % slower at
