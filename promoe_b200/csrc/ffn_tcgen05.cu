@@ -126,16 +126,28 @@ struct RingPos {
 
 // Group table: token tiles of equal width (a multiple of 32, at most 256) and the tile ranges.
 template <bool GATEUP>
-__device__ __forceinline__ void build_table(TcShared& sh, const TcGroup* __restrict__ groups, int n_groups, int hidden) {
+__device__ __forceinline__ void build_table(TcShared& sh, const TcGroup* __restrict__ groups, const TcPlan& plan, int n_groups,
+                                            int hidden) {
   for (int i = threadIdx.x; i < n_groups; i += blockDim.x) {
-    const TcGroup g = groups[i];
+    TcGroup g;
+    if (groups != nullptr) {
+      g = groups[i];
+    } else {  // group 0 is the shared expert where there is one, then the experts in order, absent ones with no rows
+      const int e = i - (plan.shared_inter > 0 ? 1 : 0);
+      if (e < 0) {
+        g = TcGroup{plan.n_routed_rows, plan.tokens, plan.shared_inter, -1};
+      } else {
+        const int slot = plan.slot_table[e];
+        g = TcGroup{plan.offsets[e], slot >= 0 ? plan.counts[e] : 0, plan.inter, plan.first_line + slot};
+      }
+    }
     TcSlot t;
     t.row_start = g.row_start;
     t.rows = g.row_count;
     t.line = g.line;
     t.inter = g.inter;
     t.n_tiles = (g.row_count + kTcMaxN - 1) / kTcMaxN;
-    t.width = ((g.row_count + t.n_tiles - 1) / t.n_tiles + 31) / 32 * 32;
+    t.width = t.n_tiles > 0 ? ((g.row_count + t.n_tiles - 1) / t.n_tiles + 31) / 32 * 32 : 0;
     const int m_tiles = GATEUP ? (g.inter + 127) / 128 : (hidden + 255) / 256;
     t.first_tile = t.n_tiles * m_tiles;  // a count; the scan below turns it into a position
     sh.slot[i] = t;
@@ -213,8 +225,8 @@ __device__ __forceinline__ uint32_t nibble_at(uint32_t word, uint32_t exponent) 
 template <bool GATEUP, bool Q4>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc_threads<Q4>(), 1)
 prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ TcScales scales, const TcRing ring,
-                   const TcGroup* __restrict__ groups, int n_groups, int hidden, __nv_bfloat16* __restrict__ hbuf,
-                   int ld_h, float* __restrict__ yexp, int32_t* __restrict__ err) {
+                   const TcGroup* __restrict__ groups, const TcPlan plan, int n_groups, int hidden,
+                   __nv_bfloat16* __restrict__ hbuf, int ld_h, float* __restrict__ yexp, int32_t* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
   // the same offset in both CTAs of the pair: the MMA addresses both through one descriptor
   unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -245,7 +257,7 @@ prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ 
     fence_barrier_init();
   }
   if (warp == 2) tmem_alloc(&sh.tmem_base, kTmemCols);
-  build_table<GATEUP>(sh, groups, n_groups, hidden);
+  build_table<GATEUP>(sh, groups, plan, n_groups, hidden);
   tc_fence_before();
   cluster_sync();
   tc_fence_after();
@@ -571,7 +583,7 @@ cudaError_t launch_pair(const TcLaunch& a, cudaStream_t s, cudaEvent_t mid_event
   const TcScales sc{a.scale_base, a.scale_stride, a.scale_gate, a.scale_up, a.scale_down, 0x4B000000u};
   const size_t smem = ring.smem_bytes();
   prefill_ffn_kernel<true, Q4><<<2 * std::min(pairs, a.tiles_gu), tc_threads<Q4>(), smem, s>>>(
-      *a.maps, sc, ring, a.groups_dev, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
+      *a.maps, sc, ring, a.groups_dev, a.plan, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (mid_event != nullptr) {
@@ -579,7 +591,7 @@ cudaError_t launch_pair(const TcLaunch& a, cudaStream_t s, cudaEvent_t mid_event
     if (e != cudaSuccess) return e;
   }
   prefill_ffn_kernel<false, Q4><<<2 * std::min(pairs, a.tiles_dn), tc_threads<Q4>(), smem, s>>>(
-      *a.maps, sc, ring, a.groups_dev, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
+      *a.maps, sc, ring, a.groups_dev, a.plan, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
   return cudaGetLastError();
 }
 

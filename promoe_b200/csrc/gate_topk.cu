@@ -312,6 +312,7 @@ route_small_kernel(const __grid_constant__ RouteArgs a) {
   __syncthreads();
   for (int i = tid; i < E; i += kRouteThreads) a.counts[i] = cnt[i];
   for (int i = tid; i <= E; i += kRouteThreads) a.offsets[i] = off[i];
+  for (int i = off[E] + tid; i < R; i += kRouteThreads) a.row_token[i] = 0;  // rows that no pair takes
   if (e >= 0) {
     const int p = off[e] + before;
     a.row_token[p] = tid / k;

@@ -102,6 +102,8 @@ permute_kernel(const int32_t* __restrict__ topk_ids, int R, int k, int E, int32_
   __syncthreads();
   for (int e = tid; e < E; e += kPermThreads) counts[e] = cnt[e];
   for (int e = tid; e <= E; e += kPermThreads) offsets[e] = base[e];
+  // rows that no pair takes (dropped pairs) read token 0, not what an earlier call left there
+  for (int i = base[E] + tid; i < R; i += kPermThreads) row_token[i] = 0;
   for (int i0 = 0; i0 < R; i0 += kPermThreads)
     place_pairs(i0 + tid, expert_of(topk_ids, i0 + tid, R, E, nullptr), k, E, base, wcnt, row_token, pos);
 }
@@ -151,6 +153,7 @@ permute_place_kernel(const int32_t* __restrict__ topk_ids, int R, int k, int E, 
   if (blockIdx.x == 0) {
     for (int e = tid; e < E; e += kPermThreads) counts[e] = tot[e];
     for (int e = tid; e <= E; e += kPermThreads) offsets[e] = base[e];
+    for (int i = base[E] + tid; i < R; i += kPermThreads) row_token[i] = 0;  // rows that no pair takes
     __syncthreads();
   }
   if (tid < E) base[tid] += mine[tid];

@@ -125,6 +125,7 @@ constexpr int kMaxFusedGroupsQ4 = 128;                    // same for uint4 expe
 // The shared expert is cut along its intermediate dimension into slices of `shared_slice` columns,
 // each a group of its own with its own output rows (the combine adds them), so that every tile
 // of the launch has about the same weight bytes.
+// An expert (or slice) with more than chunk_rows rows becomes several chunks.
 struct ResidentArgs {
   const int32_t* counts;      // [num_expert] routed rows per expert (permutation output)
   const int32_t* offsets;     // [num_expert + 1]
@@ -132,10 +133,23 @@ struct ResidentArgs {
   const unsigned char* pool_base;  // first cache line of the layer's pool
   size_t line_stride;
   size_t off_gate, off_up, off_down;  // tensor offsets inside a line
+  size_t off_qgate, off_qup, off_qdown;  // uint4 experts: scale / zero tensors
   const void *shared_w_gate, *shared_w_up, *shared_w_down;
   int32_t num_expert, inter, shared_inter, shared_slice;
   int32_t tokens, n_routed_rows;
+  int32_t chunk_rows, quant4;
 };
+// Rows per chunk of such a launch when an expert may have up to row_bound rows. bf16: the kernel variant for 8 rows
+// or the one for 16. uint4: chunks of 8, the unpacking limits that kernel and its 16-row variant takes 1.6
+// times as long per chunk, so an expert of 9-16 rows (unpacked twice) is the smaller cost.
+inline int resident_chunk_rows(int row_bound, int quant4) { return quant4 || row_bound <= 8 ? 8 : 16; }
+// Most chunks such a launch can have.
+inline int resident_max_chunks(const ResidentArgs& a, int row_bound) {
+  const int per = (row_bound + a.chunk_rows - 1) / a.chunk_rows;
+  const int routed = a.n_routed_rows / a.chunk_rows + a.num_expert;
+  const int slices = a.shared_inter > 0 ? (a.shared_inter + a.shared_slice - 1) / a.shared_slice : 0;
+  return (routed < per * a.num_expert ? routed : per * a.num_expert) + slices * ((a.tokens + a.chunk_rows - 1) / a.chunk_rows);
+}
 // Width of one slice of a shared expert of width shared_inter beside routed experts of width inter.
 inline int shared_slice_width(int inter, int shared_inter) {
   int w = inter > 0 ? inter : shared_inter;
@@ -151,12 +165,12 @@ inline int shared_slice_count(int inter, int shared_inter) {
 }
 // Launches the fused FFN for the shared expert (sliced) and every activated resident expert.
 // counters: kMaxFusedGroups + 1 int32 (per chunk, then the launch total), zero at launch. err: a device word that receives a non-zero
-// code if a bounded dependency wait gives up. Needs cooperative launch and at most kSplitMaxRows
-// rows per expert.
-cudaError_t launch_resident_ffn(const ResidentArgs& a, int32_t* counters, int32_t* err, int max_rows,
+// code if a bounded dependency wait gives up. Needs cooperative launch and resident_max_chunks within the kernel's
+// table (kMaxFusedGroups, uint4: kMaxFusedGroupsQ4).
+cudaError_t launch_resident_ffn(const ResidentArgs& a, int32_t* counters, int32_t* err,
                                 const __nv_bfloat16* x, int hidden, const int32_t* row_token,
                                 __nv_bfloat16* hbuf, int ld_h, float* yexp, cudaStream_t s);
-bool resident_ffn_available(int max_rows);
+bool resident_ffn_available(int chunk_rows, int quant4);
 
 // Launches of at most kSplitMaxRows rows per chunk run as ONE cooperative kernel (gate/up tiles,
 // then down tiles, a chunk's down tiles waiting on its gate/up tiles through the blob's counters),
@@ -194,12 +208,20 @@ struct TcGroup {
   int32_t row_start, row_count, inter;
   int32_t line;  // global cache line of the expert, -1 = the shared expert
 };
+// The groups of a launch pair as the device knows them behind the router: the shared expert (if any) and every
+// activated expert the layer's slot table shows resident.
+struct TcPlan {
+  const int32_t *counts, *offsets, *slot_table;
+  int32_t num_expert, first_line;  // first_line: global cache line of slot 0
+  int32_t inter, shared_inter, tokens, n_routed_rows;
+};
 constexpr int kTcMaxN = 256;       // token rows per tile
 constexpr int kMaxTcGroups = 264;  // groups of one launch pair (every expert and the shared one)
 struct TcLaunch {
   const TcMaps* maps;
-  const TcGroup* groups_dev;
-  int n_groups, max_rows;      // groups, rows of the largest
+  const TcGroup* groups_dev;   // nullptr: the groups of `plan`
+  TcPlan plan;
+  int n_groups, max_rows;      // groups, rows of the largest (with a plan: bounds)
   int tiles_gu, tiles_dn;      // tiles of the two launches (tc_tile_count), which bound their grids
   int hidden, ld_h;
   __nv_bfloat16* hbuf;

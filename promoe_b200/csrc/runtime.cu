@@ -535,11 +535,8 @@ struct PendingForward {
 
 namespace {
 
-// Groups on the tcgen05 path: gather the token rows once per layer call, upload the groups, launch the
-// gate/up and the down kernel. All groups are of one kind: uint4 experts (q4), which the kernel expands
-// to bf16 on their way into shared memory, or bf16 (experts and the shared expert).
-int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows,
-                     cudaStream_t s, bool q4) {
+// Once per layer call before its first tensor-core launch: the token rows in expert order, the tensor maps.
+int tc_prepare(pm_ctx* c, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows, cudaStream_t s) {
   if (!c->xperm_ready) {
     PM_CUDA(launch_gather_rows(x, c->d_row_token, n_rows, (size_t)w.hidden * 2, c->d_xperm, s));
     c->kernel_launches += 1;
@@ -549,6 +546,36 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
     int rc = tc_build_maps(c, w, c->ws_tokens * (c->ws_topk + 1), &c->tc_maps);
     if (rc != PM_OK) return rc;
     c->tc_maps_ready = true;
+  }
+  return PM_OK;
+}
+
+TcLaunch tc_launch_args(pm_ctx* c, const pm_layer_weights& w, bool q4) {
+  TcLaunch a{};
+  a.maps = &c->tc_maps;
+  a.hidden = w.hidden;
+  a.ld_h = c->ws_inter;
+  a.hbuf = c->d_hbuf;
+  a.yexp = c->d_yexp;
+  a.err_dev = c->d_tc_err;
+  if (q4) {
+    a.scale_base = c->slab;
+    a.scale_stride = c->line_stride;
+    a.scale_gate = c->param_offset[c->role_qgate];
+    a.scale_up = c->param_offset[c->role_qup];
+    a.scale_down = c->param_offset[c->role_qdown];
+  }
+  return a;
+}
+
+// Groups on the tcgen05 path: upload the groups, launch the
+// gate/up and the down kernel. All groups are of one kind: uint4 experts (q4), which the kernel expands
+// to bf16 on their way into shared memory, or bf16 (experts and the shared expert).
+int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows,
+                     cudaStream_t s, bool q4) {
+  {
+    int rc = tc_prepare(c, w, x, n_rows, s);
+    if (rc != PM_OK) return rc;
   }
   std::vector<TcGroup> groups;
   int max_rows = 0;
@@ -580,25 +607,12 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
     }
     PM_CUDA(cudaEventRecord(sample.e0, s));
   }
-  TcLaunch a{};
-  a.maps = &c->tc_maps;
+  TcLaunch a = tc_launch_args(c, w, q4);
   a.groups_dev = (const TcGroup*)d;
   a.n_groups = (int)groups.size();
   a.max_rows = max_rows;
   a.tiles_gu = tiles_gu;
   a.tiles_dn = tiles_dn;
-  a.hidden = w.hidden;
-  a.ld_h = c->ws_inter;
-  a.hbuf = c->d_hbuf;
-  a.yexp = c->d_yexp;
-  a.err_dev = c->d_tc_err;
-  if (q4) {
-    a.scale_base = c->slab;
-    a.scale_stride = c->line_stride;
-    a.scale_gate = c->param_offset[c->role_qgate];
-    a.scale_up = c->param_offset[c->role_qup];
-    a.scale_down = c->param_offset[c->role_qdown];
-  }
   PM_CUDA(launch_prefill_ffn(a, s, c->profile_ffn ? sample.e1 : nullptr));
   if (c->profile_ffn) {
     PM_CUDA(cudaEventRecord(sample.e2, s));
@@ -840,6 +854,59 @@ int finish_forward(pm_ctx* c, PendingForward& p) {
 
 }  // namespace
 
+namespace {
+
+// The launch for the shared expert and the experts already resident, enqueued behind the router without waiting for
+// the host to read the row counts (25 to 35 us of an idle GPU per layer call otherwise).
+enum class DevicePlan { kNone, kSplit, kTc };
+
+// Which kernel it uses has to follow from the sizes alone:
+//  bf16   up to 32 rows per expert the split-K kernel, as flush_segment chooses; above, a shared expert (T rows) would
+//         take the call to the tensor cores, and so do 16 rows per expert on average without one
+//  uint4  up to 8 rows per expert on average split-K chunks, from 24 on the tensor cores (q4_prefers_tc's line lies
+//         at about 16)
+// and what is in between waits for the counts. A bf16 shared expert beside uint4 experts does too, and so do
+// caller-routed rows that could be many: most of those may be padding.
+DevicePlan choose_device_plan(pm_ctx* c, int layer, const pm_layer_weights& w, bool has_shared, bool sliced, bool routed,
+                              int T, int R, int row_bound, ResidentArgs* a) {
+  if (!c->device_plan || (w.quant4 && has_shared)) return DevicePlan::kNone;
+  const int E = c->cfg.num_expert;
+  const Pool& pool = c->eng->pools()[c->eng->pool_index(layer)];
+  a->counts = c->d_counts;
+  a->offsets = c->d_offsets;
+  a->slot_table = c->layers[layer].slot_table_dev;
+  a->pool_base = line_ptr(c, pool.base);
+  a->line_stride = c->line_stride;
+  a->off_gate = c->param_offset[c->role_gate];
+  a->off_up = c->param_offset[c->role_up];
+  a->off_down = c->param_offset[c->role_down];
+  if (w.quant4) {
+    a->off_qgate = c->param_offset[c->role_qgate];
+    a->off_qup = c->param_offset[c->role_qup];
+    a->off_qdown = c->param_offset[c->role_qdown];
+  }
+  a->shared_w_gate = w.shared_w_gate;
+  a->shared_w_up = w.shared_w_up;
+  a->shared_w_down = w.shared_w_down;
+  a->num_expert = E;
+  a->inter = w.inter;
+  a->shared_inter = has_shared ? w.shared_inter : 0;
+  a->shared_slice = !has_shared ? 0 : sliced ? shared_slice_width(w.inter, w.shared_inter) : w.shared_inter;
+  a->tokens = T;
+  a->n_routed_rows = R;
+  a->quant4 = w.quant4;
+  a->chunk_rows = resident_chunk_rows(row_bound, w.quant4);
+  const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w) && (!has_shared || tc_shared_usable(w));
+  const bool split = w.quant4 ? R <= 8 * E || !tc_ok : row_bound <= kSplitChunkedMaxRows;
+  const bool tc = tc_ok && !routed && (w.quant4 ? R >= 24 * E : row_bound > kSplitChunkedMaxRows && (has_shared || R >= 16 * E));
+  if (split && resident_ffn_available(a->chunk_rows, w.quant4) &&
+      resident_max_chunks(*a, row_bound) <= (w.quant4 ? kMaxFusedGroupsQ4 : kMaxFusedGroups))
+    return DevicePlan::kSplit;
+  return tc ? DevicePlan::kTc : DevicePlan::kNone;
+}
+
+}  // namespace
+
 int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream_t s, const RoutedRows* routed) {
   if (!c->slab_built) return fail(PM_ERR_STATE, "moe_forward before build_slab");
   if (layer < 0 || layer >= c->cfg.num_layer) return fail(PM_ERR_INVALID, "layer out of range");
@@ -867,6 +934,8 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   c->have_last_stream = true;
   const __nv_bfloat16* x = (const __nv_bfloat16*)xv;
   Stage st = stage_of(c);
+  c->xperm_ready = false;
+  c->tc_maps_ready = false;
 
   // Refresh this layer's expert -> slot table if the cache changed since the last upload.
   if (ly.slot_table_dirty) {
@@ -876,8 +945,10 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   }
   // rows per expert <= T, or the bound the caller of the routed-rows form guarantees
   const int row_bound = (routed && routed->max_rows_per_expert > 0) ? std::min(T, routed->max_rows_per_expert) : T;
-  const bool spec = c->device_plan && !w.quant4 && resident_ffn_available(row_bound);
-  int32_t* zero_words = spec ? c->d_res_counters : nullptr;
+  ResidentArgs res{};
+  const DevicePlan plan = choose_device_plan(c, layer, w, has_shared, sliced, routed != nullptr, T, R, row_bound, &res);
+  const bool spec = plan != DevicePlan::kNone;
+  int32_t* zero_words = plan == DevicePlan::kSplit ? c->d_res_counters : nullptr;
   if (!routed && route_small_usable(T, H)) {
     RouteArgs a{};
     a.x = x; a.w_gate = (const __nv_bfloat16*)w.gate_w; a.bias = w.gate_bias;
@@ -887,7 +958,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
     a.topk_ids = c->d_topk_ids; a.topk_w = c->d_topk_w; a.topk_slot = c->d_topk_slot; a.shared_scale = c->d_shared_scale;
     a.counts = c->d_counts; a.offsets = c->d_offsets; a.row_token = c->d_row_token; a.pos = c->d_pos; a.err_flag = c->d_err;
     a.tail_rows = n_shared * T;
-    a.zero_words = zero_words; a.zero_n = spec ? kMaxFusedGroups + 1 : 0;
+    a.zero_words = zero_words; a.zero_n = zero_words != nullptr ? kMaxFusedGroups + 1 : 0;
     PM_CUDA(launch_route_small(a, s));
     c->kernel_launches += 1;
   } else {
@@ -969,6 +1040,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
 
   // Experts resident right now (the device slot table shows the same state).
   std::vector<int> resident_line(E, -1);
+  std::vector<cudaEvent_t> read_before(E, nullptr);
   pm_ctx::FfnSample spec_sample{};
   if (spec) {
     for (int e = 0; e < E; ++e) {
@@ -981,25 +1053,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
         c->line_waiter[line] = s;
       }
     }
-    ResidentArgs a{};
-    const Pool& pool = c->eng->pools()[c->eng->pool_index(layer)];
-    a.counts = c->d_counts;
-    a.offsets = c->d_offsets;
-    a.slot_table = ly.slot_table_dev;
-    a.pool_base = line_ptr(c, pool.base);
-    a.line_stride = c->line_stride;
-    a.off_gate = c->param_offset[c->role_gate];
-    a.off_up = c->param_offset[c->role_up];
-    a.off_down = c->param_offset[c->role_down];
-    a.shared_w_gate = w.shared_w_gate;
-    a.shared_w_up = w.shared_w_up;
-    a.shared_w_down = w.shared_w_down;
-    a.num_expert = E;
-    a.inter = w.inter;
-    a.shared_inter = has_shared ? w.shared_inter : 0;
-    a.shared_slice = has_shared ? shared_slice_width(w.inter, w.shared_inter) : 0;
-    a.tokens = T;
-    a.n_routed_rows = R;
+    const bool tc = plan == DevicePlan::kTc;
     if (c->profile_ffn) {
       auto take_event = [&](cudaEvent_t* e) -> cudaError_t {
         if (!c->ffn_event_pool.empty()) {
@@ -1009,28 +1063,45 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
         }
         return cudaEventCreate(e);
       };
-      spec_sample.fused = true;
+      spec_sample.fused = !tc;
       spec_sample.resident = true;
       PM_CUDA(take_event(&spec_sample.e0));
+      if (tc) PM_CUDA(take_event(&spec_sample.e1));
       PM_CUDA(take_event(&spec_sample.e2));
-      PM_CUDA(cudaEventRecord(spec_sample.e0, s));
     }
-    PM_CUDA(launch_resident_ffn(a, c->d_res_counters, c->d_tc_err, row_bound, x, H, c->d_row_token, c->d_hbuf,
-                                c->ws_inter, c->d_yexp, s));
+    if (tc) {
+      rc = tc_prepare(c, w, x, R + n_shared * T, s);
+      if (rc != PM_OK) return rc;
+      if (c->profile_ffn) PM_CUDA(cudaEventRecord(spec_sample.e0, s));
+      TcLaunch a = tc_launch_args(c, w, w.quant4 != 0);
+      a.groups_dev = nullptr;
+      a.plan = TcPlan{res.counts, res.offsets, res.slot_table, E, c->eng->pools()[c->eng->pool_index(layer)].base,
+                      w.inter, res.shared_inter, T, R};
+      a.n_groups = E + (has_shared ? 1 : 0);
+      a.max_rows = row_bound;
+      a.tiles_gu = a.tiles_dn = 1 << 20;  // only known on the device: full grids
+      PM_CUDA(launch_prefill_ffn(a, s, c->profile_ffn ? spec_sample.e1 : nullptr));
+      c->kernel_launches += 2;
+      c->tc_launches += 1;
+    } else {
+      if (c->profile_ffn) PM_CUDA(cudaEventRecord(spec_sample.e0, s));
+      PM_CUDA(launch_resident_ffn(res, c->d_res_counters, c->d_tc_err, x, H, c->d_row_token, c->d_hbuf, c->ws_inter, c->d_yexp, s));
+      c->kernel_launches += 1;
+    }
     if (c->profile_ffn) PM_CUDA(cudaEventRecord(spec_sample.e2, s));
-    c->kernel_launches += 1;
     cudaEvent_t ev = next_seg_event(c);
     PM_CUDA(cudaEventRecord(ev, s));
     for (int e = 0; e < E; ++e)
-      if (resident_line[e] >= 0) c->line_read[resident_line[e]] = ev;
+      if (resident_line[e] >= 0) {
+        read_before[e] = c->line_read[resident_line[e]];
+        c->line_read[resident_line[e]] = ev;
+      }
   }
   rc = wait_event(c->sync_event, 30.0);
   if (rc != PM_OK) return rc;
   // everything enqueued by earlier layer calls has finished: the staging buffers may be reused, and
   // an error the prefill kernel of an earlier call recorded is visible now
   c->tc_plan_used = 0;
-  c->xperm_ready = false;
-  c->tc_maps_ready = false;
   if (c->profile_ffn && !c->ffn_samples.empty()) {  // their events have fired: recycle them now
     rc = rt_profile_collect(c);
     if (rc != PM_OK) return rc;
@@ -1049,6 +1120,12 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
     PM_CUDA(cudaMemsetAsync(c->d_err, 0, 4, s));
     return fail(PM_ERR_INVALID, "an expert id outside [0, num_expert) was passed for a routed row");
   }
+  // The device-planned launch reads the lines of the activated experts only: a copy into another line (a victim is
+  // usually one) need not wait for it.
+  const int32_t* counts = st.counts;
+  if (spec)
+    for (int e = 0; e < E; ++e)
+      if (resident_line[e] >= 0 && counts[e] == 0) c->line_read[resident_line[e]] = read_before[e];
   if (keep) {
     c->last_ids[layer].assign(st.ids, st.ids + R);
     c->last_w[layer].assign(st.w, st.w + R);
@@ -1071,7 +1148,6 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
       if (rc != PM_OK) return rc;
     }
 
-  const int32_t* counts = st.counts;
   const int32_t* offsets = st.counts + E;
   std::vector<int64_t> ids;
   for (int e = 0; e < E; ++e)
@@ -1087,14 +1163,18 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   }
   rt_mark_dirty(c, acts);
 
-  if (spec && c->profile_ffn) {  // weight bytes the device-planned launch read: shared + activated residents
-    const int64_t routed = (int64_t)w.inter * H * 2, sh = (int64_t)w.shared_inter * H * 2;
+  if (spec && (c->profile_ffn || (plan == DevicePlan::kTc && w.quant4))) {
     int64_t n_res = 0;
     for (int e = 0; e < E; ++e)
       if (counts[e] > 0 && resident_line[e] >= 0) ++n_res;
-    spec_sample.bytes_gu = 2 * (n_res * routed + sh);
-    spec_sample.bytes_dn = n_res * routed + sh;
-    c->ffn_samples.push_back(spec_sample);
+    if (plan == DevicePlan::kTc && w.quant4) c->q4_expanded += n_res;
+    if (c->profile_ffn) {  // weight bytes the device-planned launch read: shared + activated residents
+      const int64_t mat = (int64_t)w.inter * H, sh = has_shared ? (int64_t)w.shared_inter * H * 2 : 0;
+      const int64_t one = w.quant4 ? mat / 2 + mat / 128 * 4 : mat * 2;
+      spec_sample.bytes_gu = 2 * (n_res * one + sh);
+      spec_sample.bytes_dn = n_res * one + sh;
+      c->ffn_samples.push_back(spec_sample);
+    }
   }
 
   PendingForward& p = *c->pending;

@@ -835,32 +835,30 @@ __device__ __forceinline__ void build_chunk_table(const FusedLaunch& a, G* sg, i
     }
     return;
   }
-  if constexpr (Q4) {  // uint4 launches are always host-planned
-    if (threadIdx.x == 0) meta[0] = meta[1] = meta[2] = 0;
-    return;
-  }
   const ResidentArgs& r = a.res;
   const int dn_tiles = a.hidden / kSplitTileDn;
   const int slice = r.shared_slice;
-  const int n_sh = r.shared_inter > 0 ? (r.shared_inter + slice - 1) / slice : 0;
-  const int sh_tiles = r.shared_inter / kSplitTileGu;
-  if ((int)threadIdx.x < n_sh) {  // heaviest rows first: the slices of the shared expert
-    const int j = threadIdx.x;
+  // the shared expert: slices of its width, each over all tokens, which are cut into chunks (several slices only
+  // for batches of one chunk)
+  const int sh_chunks = (r.tokens + r.chunk_rows - 1) / r.chunk_rows;
+  const int n_sh = r.shared_inter > 0 ? (r.shared_inter + slice - 1) / slice * sh_chunks : 0;
+  const int sh_tiles = r.shared_inter / kSplitTileGu * sh_chunks;
+  if (!Q4 && (int)threadIdx.x < n_sh) {  // heaviest rows first
+    const int j = threadIdx.x / sh_chunks, c = threadIdx.x - j * sh_chunks;
     G g{};
     g.w_gate = reinterpret_cast<const unsigned char*>(r.shared_w_gate) + (size_t)j * slice * a.hidden * 2;
     g.w_up = reinterpret_cast<const unsigned char*>(r.shared_w_up) + (size_t)j * slice * a.hidden * 2;
     g.w_down = reinterpret_cast<const unsigned char*>(r.shared_w_down) + (size_t)j * slice * 2;
-    g.row_start = r.n_routed_rows + j * r.tokens;
-    g.rows = r.tokens;
+    g.row_start = r.n_routed_rows + j * r.tokens + c * r.chunk_rows;
+    g.rows = min(r.chunk_rows, r.tokens - c * r.chunk_rows);
     g.inter = min(slice, r.shared_inter - j * slice);
     g.ld_down = r.shared_inter;
-    g.tile_gu = j * (slice / kSplitTileGu);
-    g.tile_dn = j * dn_tiles;
-    sg[j] = g;
+    g.tile_gu = (int)threadIdx.x * (slice / kSplitTileGu);
+    g.tile_dn = (int)threadIdx.x * dn_tiles;
+    sg[threadIdx.x] = g;
   }
-  if (threadIdx.x < 32) {  // one warp compacts the activated resident experts in ascending id order
+  if (threadIdx.x < 32) {  // one warp lists the chunks of the activated resident experts in ascending id order
     const int lane = threadIdx.x;
-    const unsigned lt = (1u << lane) - 1u;
     const int gu_tiles = r.inter / kSplitTileGu;
     int base = n_sh;
     for (int c = 0; c < r.num_expert; c += 32) {
@@ -871,24 +869,34 @@ __device__ __forceinline__ void build_chunk_table(const FusedLaunch& a, G* sg, i
         slot = r.slot_table[e];
         off = r.offsets[e];
       }
-      const bool act = cnt > 0 && slot >= 0;
-      const unsigned mask = __ballot_sync(0xffffffffu, act);
-      if (act) {
-        const int idx = base + __popc(mask & lt);
-        const unsigned char* line = r.pool_base + (size_t)slot * r.line_stride;
+      const int n = slot >= 0 ? (cnt + r.chunk_rows - 1) / r.chunk_rows : 0;
+      int incl = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+      }
+      const unsigned char* line = r.pool_base + (size_t)(slot < 0 ? 0 : slot) * r.line_stride;
+      for (int k = 0; k < n; ++k) {
+        const int idx = base + incl - n + k;
         G g{};
+        if constexpr (Q4) {
+          g.q_gate = reinterpret_cast<const uint32_t*>(line + r.off_qgate);
+          g.q_up = reinterpret_cast<const uint32_t*>(line + r.off_qup);
+          g.q_down = reinterpret_cast<const uint32_t*>(line + r.off_qdown);
+        }
         g.w_gate = line + r.off_gate;
         g.w_up = line + r.off_up;
         g.w_down = line + r.off_down;
-        g.row_start = off;
-        g.rows = cnt;
+        g.row_start = off + k * r.chunk_rows;
+        g.rows = min(r.chunk_rows, cnt - k * r.chunk_rows);
         g.inter = r.inter;
         g.ld_down = r.inter;
         g.tile_gu = sh_tiles + (idx - n_sh) * gu_tiles;
         g.tile_dn = idx * dn_tiles;
         sg[idx] = g;
       }
-      base += __popc(mask);
+      base += __shfl_sync(0xffffffffu, incl, 31);
     }
     if (lane == 0) {
       meta[0] = base;
@@ -1005,10 +1013,9 @@ cudaError_t dispatch_nt(int max_rows, const GroupDesc* groups, const int32_t* ti
 
 }  // namespace
 
-cudaError_t launch_resident_ffn(const ResidentArgs& r, int32_t* counters, int32_t* err, int max_rows,
+cudaError_t launch_resident_ffn(const ResidentArgs& r, int32_t* counters, int32_t* err,
                                 const __nv_bfloat16* x, int hidden, const int32_t* row_token,
                                 __nv_bfloat16* hbuf, int ld_h, float* yexp, cudaStream_t s) {
-  if (max_rows > kSplitMaxRows) return cudaErrorNotSupported;
   FusedLaunch a{};
   a.groups = nullptr;
   a.res = r;
@@ -1021,12 +1028,13 @@ cudaError_t launch_resident_ffn(const ResidentArgs& r, int32_t* counters, int32_
   a.yexp = yexp;
   a.hidden = hidden;
   a.ld_h = ld_h;
-  return launch_fused_rows(a, max_rows, 0, s);  // the tile count is only known on the device: full grid
+  // the tile count is only known on the device: full grid
+  return r.quant4 ? launch_fused_rows_q4(a, r.chunk_rows, 0, s) : launch_fused_rows(a, r.chunk_rows, 0, s);
 }
 
-bool resident_ffn_available(int max_rows) {
-  if (max_rows > kSplitMaxRows) return false;
-  return (max_rows <= 8 ? fused_grid_size<1, 4, false>() : fused_grid_size<2, 2, false>()) > 0;
+bool resident_ffn_available(int chunk_rows, int quant4) {
+  if (quant4) return fused_grid_size<1, 2, true>() > 0;
+  return (chunk_rows <= 8 ? fused_grid_size<1, 4, false>() : fused_grid_size<2, 2, false>()) > 0;
 }
 
 cudaError_t launch_swiglu_ffn(const unsigned char* blob_dev, const FfnPlanInfo& info, int quant4,
