@@ -524,8 +524,15 @@ __device__ __forceinline__ void tile_issue_a(const TileCtx<NT>& t, int s0, uint4
 }
 
 template <int NT, int DEPTH, bool COHERENT_B, bool Q4, int FIRST = 0, int COUNT = DEPTH>
-__device__ __forceinline__ void tile_issue_b(const TileCtx<NT>& t, int s0, uint4 (&b)[DEPTH][NT]) {
-  if constexpr (!Q4) {  // uint4 tiles fetch their token values (L1/L2 hits) inside tile_compute_q4
+__device__ __forceinline__ void tile_issue_b(const TileCtx<NT>& t, int s0, uint4 (&b)[DEPTH][NT], uint4 (&bq)[NT][4]) {
+  if constexpr (Q4) {  // the first step's token values; tile_compute_q4 fetches each later step's one step ahead
+    if (FIRST == 0 && s0 < t.s_end) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) bq[nt][v] = load_b<COHERENT_B>(t.b_ptr[nt] + (size_t)s0 * 256 + v * 16);
+    }
+  } else {
 #pragma unroll
     for (int d = FIRST; d < FIRST + COUNT; ++d) {
       if (s0 + d < t.s_end) {
@@ -562,7 +569,8 @@ __device__ __forceinline__ void tile_compute(const TileCtx<NT>& t, int s0, const
 // (see the layout note above q4_pair), then the per-group scale / zero fix-up.
 template <int NT, int DEPTH, bool COHERENT_B, int FIRST = 0, int COUNT = DEPTH>
 __device__ __forceinline__ void tile_compute_q4(const TileCtx<NT>& t, int s0, const uint4 (&a)[DEPTH][4],
-                                                const uint32_t (&sz)[DEPTH][4], float (&acc)[2][NT][4], uint32_t ex) {
+                                                const uint32_t (&sz)[DEPTH][4], float (&acc)[2][NT][4], uint32_t ex,
+                                                uint4 (&bq)[NT][4]) {
   constexpr uint32_t kOnes = 0x3F803F80u;  // bf16 (1, 1)
 #pragma unroll
   for (int d = FIRST; d < FIRST + COUNT; ++d) {
@@ -578,8 +586,13 @@ __device__ __forceinline__ void tile_compute_q4(const TileCtx<NT>& t, int s0, co
         const uint32_t w10 = (&a[d][2].x)[v], w11 = (&a[d][3].x)[v];  // second pair
         uint4 bv[NT];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-          bv[nt] = load_b<COHERENT_B>(t.b_ptr[nt] + (size_t)(s0 + d) * 256 + v * 16);
+        for (int nt = 0; nt < NT; ++nt) {
+          bv[nt] = bq[nt][v];
+          // the next step's token values, a whole step ahead of their use: out of L1 / L2 they take 300 cycles and
+          // more (8 experts of 4096 x 14336, 16 tokens: 215 us when they were loaded where they are used, 200 us)
+          if (s0 + d + 1 < t.s_end)
+            bq[nt][v] = load_b<COHERENT_B>(t.b_ptr[nt] + (size_t)(s0 + d + 1) * 256 + v * 16);
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {  // nibble pairs {0,1} go with b.x, b.y; pairs {2,3} with b.z, b.w
           // each word is unpacked once and used for every n-tile
@@ -707,6 +720,7 @@ struct StreamState {
   uint4 a[DEPTH][4];
   uint4 b[DEPTH][NT];      // bf16 tiles only
   uint32_t sz[DEPTH][4];   // uint4 tiles only
+  uint4 bq[NT][4];         // uint4 tiles only: token values of the next step
   int tile, buf;
   bool active, all_done;
 };
@@ -752,7 +766,7 @@ __device__ __forceinline__ void stream_run(StreamState<NT, DEPTH>& st, const G* 
   // arrivals a chunk's counter shows when its intermediate rows are complete
   auto target_of = [&](int gi) { return sg[gi].inter / kSplitTileGu; };
   if (!GATEUP) wait_rows_ready(counters, total, t.gi, target_of(t.gi), total_target, st.all_done, err);
-  tile_issue_b<NT, DEPTH, COH, Q4>(t, 0, st.b);
+  tile_issue_b<NT, DEPTH, COH, Q4>(t, 0, st.b, st.bq);
   const int stride = gridDim.x;
   int next = st.tile + stride;
   int pending = -1;  // chunk of the gate/up tile whose arrival is still to be signalled
@@ -765,22 +779,22 @@ __device__ __forceinline__ void stream_run(StreamState<NT, DEPTH>& st, const G* 
     // with the steps DEPTH further on, so a warp always has loads outstanding while it waits.
     constexpr int HALF = DEPTH / 2;
     for (int s0 = 0; s0 < t.s_end; s0 += DEPTH) {
-      if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, 0, HALF>(t, s0, st.a, st.sz, acc, ex);
+      if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, 0, HALF>(t, s0, st.a, st.sz, acc, ex, st.bq);
       else tile_compute<NT, DEPTH, 0, HALF>(t, s0, st.a, st.b, acc);
       if (s0 + DEPTH < t.s_end) {
         tile_issue_a<NT, DEPTH, Q4, 0, HALF>(t, s0 + DEPTH, st.a, st.sz);
-        tile_issue_b<NT, DEPTH, COH, Q4, 0, HALF>(t, s0 + DEPTH, st.b);
+        if constexpr (!Q4) tile_issue_b<NT, DEPTH, COH, Q4, 0, HALF>(t, s0 + DEPTH, st.b, st.bq);
       }
       if (has_next && !rows_loaded) {  // fetch the next tile's token row numbers under this tile's loads
         load_src_rows<NT, GATEUP>(src_row, sg[gi_next], row_token);
         rows_loaded = true;
       }
       if (s0 + HALF < t.s_end) {
-        if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, HALF, HALF>(t, s0, st.a, st.sz, acc, ex);
+        if constexpr (Q4) tile_compute_q4<NT, DEPTH, COH, HALF, HALF>(t, s0, st.a, st.sz, acc, ex, st.bq);
         else tile_compute<NT, DEPTH, HALF, HALF>(t, s0, st.a, st.b, acc);
         if (s0 + DEPTH + HALF < t.s_end) {
           tile_issue_a<NT, DEPTH, Q4, HALF, HALF>(t, s0 + DEPTH, st.a, st.sz);
-          tile_issue_b<NT, DEPTH, COH, Q4, HALF, HALF>(t, s0 + DEPTH, st.b);
+          if constexpr (!Q4) tile_issue_b<NT, DEPTH, COH, Q4, HALF, HALF>(t, s0 + DEPTH, st.b, st.bq);
         }
       }
     }
@@ -790,7 +804,7 @@ __device__ __forceinline__ void stream_run(StreamState<NT, DEPTH>& st, const G* 
       if (!GATEUP) wait_rows_ready(counters, total, gi_next, target_of(gi_next), total_target, st.all_done, err);
       tile_setup<NT, GATEUP, WARPS>(t, sg[gi_next], gi_next, next, src_row, bsrc, ldb, hidden);
       tile_issue_a<NT, DEPTH, Q4>(t, 0, st.a, st.sz);
-      tile_issue_b<NT, DEPTH, COH, Q4>(t, 0, st.b);
+      tile_issue_b<NT, DEPTH, COH, Q4>(t, 0, st.b, st.bq);
     }
     tile_finish<NT, GATEUP, WARPS>(sg[gi], m0, acc, red2[st.buf], hbuf, ld_h, yexp, hidden, counters, total, pending);
     pending = gi;
