@@ -241,4 +241,9 @@ cudaError_t launch_predictor_mlp(const __nv_bfloat16* x, int B, int H, const __n
                                  const float* b1, int D, const __nv_bfloat16* w2, const float* b2,
                                  int E, float* hidden_scratch, float* scores, cudaStream_t s);
 
+// The same followed by launch_rank_topn on its scores, in one launch less. E at most 256.
+cudaError_t launch_predictor_ranked(const __nv_bfloat16* x, int B, int H, const __nv_bfloat16* w1, const float* b1, int D,
+                                    const __nv_bfloat16* w2, const float* b2, int E, float* hidden_scratch, float* scores,
+                                    int n, int32_t* out, cudaStream_t s);
+
 }  // namespace pm

@@ -298,17 +298,19 @@ int launch_predictors(pm_ctx* c, int src, const __nv_bfloat16* x, int B, int H, 
     const pm_ctx::Predictor& p = c->predictors[(size_t)src * L + dst];
     if (p.w1 == nullptr) continue;
     if (p.d > 4096) return fail(PM_ERR_UNSUPPORTED, "predictor hidden width above 4096");
-    PM_CUDA(launch_predictor_mlp(x, B, H, (const __nv_bfloat16*)p.w1, p.b1, p.d, (const __nv_bfloat16*)p.w2,
-                                 p.b2, E, c->d_pred_hidden, c->d_scores + (size_t)dst * E, s));
-    c->kernel_launches += 2;
     const int n = prediction_count(c, dst, E, -1);
+    float* scores = c->d_scores + (size_t)dst * E;
     if (topn_on_device(c, n, E)) {  // rank on the device: the host reads n ids instead of sorting E scores
       int rc = ensure_topn(c);
       if (rc != PM_OK) return rc;
-      PM_CUDA(launch_rank_topn(c->d_scores + (size_t)dst * E, E, n, c->d_topn + (size_t)dst * kTopCap, s));
-      c->kernel_launches += 1;
+      PM_CUDA(launch_predictor_ranked(x, B, H, (const __nv_bfloat16*)p.w1, p.b1, p.d, (const __nv_bfloat16*)p.w2, p.b2, E,
+                                      c->d_pred_hidden, scores, n, c->d_topn + (size_t)dst * kTopCap, s));
       c->topn_launches += 1;
+    } else {
+      PM_CUDA(launch_predictor_mlp(x, B, H, (const __nv_bfloat16*)p.w1, p.b1, p.d, (const __nv_bfloat16*)p.w2,
+                                   p.b2, E, c->d_pred_hidden, scores, s));
     }
+    c->kernel_launches += 2;
     dsts->push_back(dst);
   }
   return PM_OK;
