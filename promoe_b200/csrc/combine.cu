@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(kCombineThreads)
 combine_kernel(const float* __restrict__ yexp, const int32_t* __restrict__ pos,
                const float* __restrict__ topk_w, int T, int H, int k, int R, int n_shared,
                const float* __restrict__ shared_scale, __nv_bfloat16* __restrict__ y) {
+  wait_for_predecessor();
   const int t = blockIdx.x;
   __shared__ int p_s[kMaxTopK];
   __shared__ float w_s[kMaxTopK];
@@ -62,8 +63,7 @@ cudaError_t launch_combine(const float* yexp, const int32_t* pos, const float* t
                            __nv_bfloat16* y, cudaStream_t s) {
   if (T <= 0) return cudaSuccess;
   if (k > kMaxTopK) return cudaErrorInvalidValue;
-  combine_kernel<<<T, kCombineThreads, 0, s>>>(yexp, pos, topk_w, T, H, k, R, n_shared, shared_scale, y);
-  return cudaGetLastError();
+  return launch_behind(combine_kernel, T, kCombineThreads, 0, s, yexp, pos, topk_w, T, H, k, R, n_shared, shared_scale, y);
 }
 
 }  // namespace pm

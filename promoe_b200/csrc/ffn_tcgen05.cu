@@ -240,6 +240,10 @@ prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ 
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int n_stages = ring.n_stages;
 
+  // The down pass may start while the gate/up pass drains; it waits where it first needs its results (the producer
+  // of its token rows). What both read besides is complete before the gate/up pass lets it in.
+  if (GATEUP) wait_for_predecessor();
+  let_successor_start();
   if (threadIdx.x == 0) {
     for (int s = 0; s < n_stages; ++s) {
       mbar_init(&sh.full[s], 1 + (Q4 ? 2 * kDequantWarps : 0));
@@ -266,6 +270,7 @@ prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ 
 
   if (warp == 0 && lane == 0) {
     // ---- producer: this CTA's half of the weight rows (bf16 experts) and of the token rows ---------
+    if (!GATEUP) wait_for_predecessor();
     TileAt t;
     RingPos at;
     int steps = 0;
@@ -582,17 +587,15 @@ cudaError_t launch_pair(const TcLaunch& a, cudaStream_t s, cudaEvent_t mid_event
   const TcRing ring = ring_for<Q4>(a.max_rows);
   const TcScales sc{a.scale_base, a.scale_stride, a.scale_gate, a.scale_up, a.scale_down, 0x4B000000u};
   const size_t smem = ring.smem_bytes();
-  prefill_ffn_kernel<true, Q4><<<2 * std::min(pairs, a.tiles_gu), tc_threads<Q4>(), smem, s>>>(
-      *a.maps, sc, ring, a.groups_dev, a.plan, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_behind(prefill_ffn_kernel<true, Q4>, 2 * std::min(pairs, a.tiles_gu), tc_threads<Q4>(), smem, s, *a.maps,
+                                sc, ring, a.groups_dev, a.plan, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
   if (e != cudaSuccess) return e;
   if (mid_event != nullptr) {
     e = cudaEventRecord(mid_event, s);
     if (e != cudaSuccess) return e;
   }
-  prefill_ffn_kernel<false, Q4><<<2 * std::min(pairs, a.tiles_dn), tc_threads<Q4>(), smem, s>>>(
-      *a.maps, sc, ring, a.groups_dev, a.plan, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
-  return cudaGetLastError();
+  return launch_behind(prefill_ffn_kernel<false, Q4>, 2 * std::min(pairs, a.tiles_dn), tc_threads<Q4>(), smem, s, *a.maps, sc,
+                       ring, a.groups_dev, a.plan, a.n_groups, a.hidden, a.hbuf, a.ld_h, a.yexp, a.err_dev);
 }
 
 }  // namespace

@@ -171,6 +171,7 @@ gate_topk_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
                  float* __restrict__ shared_scale, float* __restrict__ logits_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];  // TOK rows of H bf16
   __shared__ float logit_all[TOK * (kMaxExperts + 1)];
+  wait_for_predecessor();
 
   const int t0 = blockIdx.x * TOK;
   const int lane = threadIdx.x & 31;
@@ -237,6 +238,7 @@ route_small_kernel(const __grid_constant__ RouteArgs a) {
   const int n_rows = E + (a.w_shared_gate != nullptr ? 1 : 0);
   const int groups = (T + TOK - 1) / TOK;
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
+  wait_for_predecessor();
 
   uint4* xs = reinterpret_cast<uint4*>(smem_raw);
   for (int idx = tid; idx < groups * TOK * nvec; idx += kRouteThreads)
@@ -333,10 +335,8 @@ cudaError_t launch_gate(const __nv_bfloat16* x, const __nv_bfloat16* w_gate, con
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<(T + TOK - 1) / TOK, warps * 32, smem, s>>>(
-      x, w_gate, bias, w_shared_gate, T, H, E, k, norm_topk, routed_scale, expert_slot, topk_ids, topk_w, topk_slot,
-      shared_scale, logits_out);
-  return cudaGetLastError();
+  return launch_behind(kern, (T + TOK - 1) / TOK, warps * 32, smem, s, x, w_gate, bias, w_shared_gate, T, H, E, k, norm_topk,
+                       routed_scale, expert_slot, topk_ids, topk_w, topk_slot, shared_scale, logits_out);
 }
 
 size_t route_small_smem(int T, int H) { return (size_t)(T > 1 ? (T + 3) / 4 * 4 : 1) * H * 2; }
@@ -352,8 +352,7 @@ cudaError_t launch_route_small(const RouteArgs& a, cudaStream_t s) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<kRouteCtas, kRouteThreads, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_behind(kern, kRouteCtas, kRouteThreads, smem, s, a);
 }
 
 cudaError_t launch_gate_topk(const __nv_bfloat16* x, const __nv_bfloat16* w_gate, const float* bias,

@@ -87,6 +87,7 @@ permute_kernel(const int32_t* __restrict__ topk_ids, int R, int k, int E, int32_
   __shared__ int cnt[kMaxExperts];
   __shared__ int base[kMaxExperts + 1];
   const int tid = threadIdx.x;
+  wait_for_predecessor();
   for (int e = tid; e < E; e += kPermThreads) cnt[e] = 0;
   for (int i = tid; i < zero_n; i += kPermThreads) zero_words[i] = 0;
   // Rows after the R routed ones belong to the shared experts: every token once per shared expert.
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(256)
 permute_count_kernel(const int32_t* __restrict__ topk_ids, int R, int E, int32_t* __restrict__ chunk_cnt,
                      int32_t* __restrict__ err_flag, int32_t* __restrict__ pos, int32_t* __restrict__ zero_words, int zero_n) {
   __shared__ int cnt[kMaxExperts];
+  wait_for_predecessor();
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < zero_n; i += blockDim.x) zero_words[i] = 0;
@@ -137,6 +139,7 @@ permute_place_kernel(const int32_t* __restrict__ topk_ids, int R, int k, int E, 
   __shared__ int tot[kMaxExperts], mine[kMaxExperts];
   __shared__ int base[kMaxExperts + 1];
   const int tid = threadIdx.x, n_chunks = gridDim.x;
+  wait_for_predecessor();
   for (int i = blockIdx.x * kPermThreads + tid; i < tail_rows; i += n_chunks * kPermThreads) row_token[R + i] = i % T;
   for (int e = tid; e < E; e += kPermThreads) tot[e] = mine[e] = 0;
   __syncthreads();
@@ -166,6 +169,7 @@ permute_place_kernel(const int32_t* __restrict__ topk_ids, int R, int k, int E, 
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ index, int n_rows, int row_vec,
                    uint4* __restrict__ dst) {
+  wait_for_predecessor();
   for (int r = blockIdx.x; r < n_rows; r += gridDim.x) {
     const int from = index[r];
     const uint4* s = src + (size_t)(from < 0 ? 0 : from) * row_vec;
@@ -180,8 +184,7 @@ cudaError_t launch_gather_rows(const void* src, const int32_t* index, int n_rows
                                cudaStream_t s) {
   if (n_rows <= 0) return cudaSuccess;
   const int grid = n_rows < 1184 ? n_rows : 1184;  // 8 x 148 SMs
-  gather_rows_kernel<<<grid, 256, 0, s>>>((const uint4*)src, index, n_rows, (int)(row_bytes / 16), (uint4*)dst);
-  return cudaGetLastError();
+  return launch_behind(gather_rows_kernel, grid, 256, 0, s, (const uint4*)src, index, n_rows, (int)(row_bytes / 16), (uint4*)dst);
 }
 
 cudaError_t launch_permute(const int32_t* topk_ids, int R, int k, int E, int32_t* counts,
@@ -192,14 +195,13 @@ cudaError_t launch_permute(const int32_t* topk_ids, int R, int k, int E, int32_t
   // Two launches cost about 4 us, every 1024 pairs in one CTA about 1.2 us.
   const int n_chunks = (R + kPermThreads - 1) / kPermThreads;
   if (n_chunks > 2 && scratch != nullptr && scratch_ints >= (size_t)n_chunks * E) {
-    permute_count_kernel<<<n_chunks, 256, 0, s>>>(topk_ids, R, E, scratch, err_flag, pos, zero_words, zero_n);
-    permute_place_kernel<<<n_chunks, kPermThreads, 0, s>>>(topk_ids, R, k, E, scratch, counts, offsets, row_token, pos,
-                                                           tail_rows, T > 0 ? T : 1);
-    return cudaGetLastError();
+    cudaError_t e = launch_behind(permute_count_kernel, n_chunks, 256, 0, s, topk_ids, R, E, scratch, err_flag, pos, zero_words, zero_n);
+    if (e != cudaSuccess) return e;
+    return launch_behind(permute_place_kernel, n_chunks, kPermThreads, 0, s, topk_ids, R, k, E, scratch, counts, offsets, row_token,
+                         pos, tail_rows, T > 0 ? T : 1);
   }
-  permute_kernel<<<1, kPermThreads, 0, s>>>(topk_ids, R, k, E, counts, offsets, row_token, pos, err_flag,
-                                            tail_rows, T > 0 ? T : 1, zero_words, zero_n);
-  return cudaGetLastError();
+  return launch_behind(permute_kernel, 1, kPermThreads, 0, s, topk_ids, R, k, E, counts, offsets, row_token, pos, err_flag, tail_rows,
+                       T > 0 ? T : 1, zero_words, zero_n);
 }
 
 }  // namespace pm

@@ -60,6 +60,30 @@ constexpr int kSplitTileDn = 32;    // or 32 down rows
 // top-6 over 64 experts lose: 155 us in chunks against 177 us.
 constexpr int kSplitChunkedMaxRows = 32;
 
+// Launches of one layer call follow each other closely: with launch_behind a kernel may be scheduled while its
+// predecessor in the stream drains (programmatic dependent launch). It has to call wait_for_predecessor before it
+// touches what earlier kernels wrote; a predecessor lets it in early with let_successor_start, in every CTA, once all
+// its own CTAs can be resident (a successor that waits may hold an SM). Walls of a pass, in turn on one GPU: one token
+// 45.9 -> 43.6 us, two layers of 8 tokens with predictors 208.9 -> 191.4, routed rows 48.4 -> 45.1, 777 tokens 312 -> 299.
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+cudaError_t launch_behind(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+#endif
+
 // Kernel launchers (defined in the .cu files). All take the caller's stream.
 cudaError_t launch_gate_topk(const __nv_bfloat16* x, const __nv_bfloat16* w_gate, const float* bias,
                              const __nv_bfloat16* w_shared_gate, int T, int H, int E, int k,

@@ -47,6 +47,7 @@ predictor_fc1_kernel(const __nv_bfloat16* __restrict__ x, int B, int H,
   extern __shared__ __align__(16) unsigned char fc1_smem[];
   uint4* xs = reinterpret_cast<uint4*>(fc1_smem);  // [kFc1Tok][H / 8]
   const int lane = threadIdx.x & 31;
+  wait_for_predecessor();
   const int j = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
   const int nvec = H / 8;
   const uint4* wrow = reinterpret_cast<const uint4*>(w1 + (size_t)min(j, D - 1) * H);
@@ -131,6 +132,7 @@ predictor_fc2_kernel(const float* __restrict__ hidden, int B, int D,
                      const __nv_bfloat16* __restrict__ w2, const float* __restrict__ b2, int E,
                      float* __restrict__ scores) {
   extern __shared__ float hsum[];  // [D]
+  wait_for_predecessor();
   sum_hidden(hidden, B, D, hsum);
   __syncthreads();
   const int e = blockIdx.x * kWarpsPerCta + (threadIdx.x >> 5);
@@ -198,6 +200,7 @@ predictor_fc2_rank_kernel(const float* __restrict__ hidden, int B, int D, const 
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(sc0) : "r"((uint32_t)__cvta_generic_to_shared(sc)));
   for (int i = threadIdx.x; i < kRankMaxExperts; i += blockDim.x) taken[i] = 0;
+  wait_for_predecessor();
   sum_hidden(hidden, B, D, hsum);
   __syncthreads();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -232,9 +235,8 @@ cudaError_t launch_fc1(const __nv_bfloat16* x, int B, int H, const __nv_bfloat16
     cudaError_t ae = cudaFuncSetAttribute(predictor_fc1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fc1_smem);
     if (ae != cudaSuccess) return ae;
   }
-  predictor_fc1_kernel<<<(D + kWarpsPerCta - 1) / kWarpsPerCta, kWarpsPerCta * 32, fc1_smem, s>>>(
-      x, B, H, w1, b1, D, hidden_scratch);
-  return cudaGetLastError();
+  return launch_behind(predictor_fc1_kernel, (D + kWarpsPerCta - 1) / kWarpsPerCta, kWarpsPerCta * 32, fc1_smem, s, x, B, H, w1,
+                       b1, D, hidden_scratch);
 }
 }  // namespace
 
@@ -244,9 +246,8 @@ cudaError_t launch_predictor_mlp(const __nv_bfloat16* x, int B, int H, const __n
   if (B <= 0) return cudaSuccess;
   cudaError_t e = launch_fc1(x, B, H, w1, b1, D, hidden_scratch, s);
   if (e != cudaSuccess) return e;
-  predictor_fc2_kernel<<<(E + kWarpsPerCta - 1) / kWarpsPerCta, kWarpsPerCta * 32, (size_t)D * 4, s>>>(
-      hidden_scratch, B, D, w2, b2, E, scores);
-  return cudaGetLastError();
+  return launch_behind(predictor_fc2_kernel, (E + kWarpsPerCta - 1) / kWarpsPerCta, kWarpsPerCta * 32, (size_t)D * 4, s,
+                       hidden_scratch, B, D, w2, b2, E, scores);
 }
 
 cudaError_t launch_predictor_ranked(const __nv_bfloat16* x, int B, int H, const __nv_bfloat16* w1, const float* b1, int D,
@@ -256,8 +257,8 @@ cudaError_t launch_predictor_ranked(const __nv_bfloat16* x, int B, int H, const 
   if (E > kRankMaxExperts || n > E) return cudaErrorInvalidValue;
   cudaError_t e = launch_fc1(x, B, H, w1, b1, D, hidden_scratch, s);
   if (e != cudaSuccess) return e;
-  predictor_fc2_rank_kernel<<<kRankCtas, kWarpsPerCta * 32, (size_t)D * 4, s>>>(hidden_scratch, B, D, w2, b2, E, scores, n, out);
-  return cudaGetLastError();
+  return launch_behind(predictor_fc2_rank_kernel, kRankCtas, kWarpsPerCta * 32, (size_t)D * 4, s, hidden_scratch, B, D, w2, b2, E,
+                       scores, n, out);
 }
 
 }  // namespace pm

@@ -1043,6 +1043,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   // Experts resident right now (the device slot table shows the same state).
   std::vector<int> resident_line(E, -1);
   std::vector<cudaEvent_t> read_before(E, nullptr);
+  bool can_evict = false;
   pm_ctx::FfnSample spec_sample{};
   if (spec) {
     for (int e = 0; e < E; ++e) {
@@ -1091,13 +1092,19 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
       c->kernel_launches += 1;
     }
     if (c->profile_ffn) PM_CUDA(cudaEventRecord(spec_sample.e2, s));
-    cudaEvent_t ev = next_seg_event(c);
-    PM_CUDA(cudaEventRecord(ev, s));
-    for (int e = 0; e < E; ++e)
-      if (resident_line[e] >= 0) {
-        read_before[e] = c->line_read[resident_line[e]];
-        c->line_read[resident_line[e]] = ev;
-      }
+    // Where the layer's pool has a line for every expert nothing is ever copied over a line that holds one, so nothing
+    // has to wait for this launch (and no event stands between it and the combine).
+    const Pool& pool = c->eng->pools()[c->eng->pool_index(layer)];
+    can_evict = !c->cfg.per_layer_cache || pool.full_len < E || c->cfg.chunk_prefetch;
+    if (can_evict) {
+      cudaEvent_t ev = next_seg_event(c);
+      PM_CUDA(cudaEventRecord(ev, s));
+      for (int e = 0; e < E; ++e)
+        if (resident_line[e] >= 0) {
+          read_before[e] = c->line_read[resident_line[e]];
+          c->line_read[resident_line[e]] = ev;
+        }
+    }
   }
   rc = wait_event(c->sync_event, 30.0);
   if (rc != PM_OK) return rc;
@@ -1125,7 +1132,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   // The device-planned launch reads the lines of the activated experts only: a copy into another line (a victim is
   // usually one) need not wait for it.
   const int32_t* counts = st.counts;
-  if (spec)
+  if (can_evict)
     for (int e = 0; e < E; ++e)
       if (resident_line[e] >= 0 && counts[e] == 0) c->line_read[resident_line[e]] = read_before[e];
   if (keep) {

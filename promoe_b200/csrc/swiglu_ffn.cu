@@ -926,6 +926,7 @@ grouped_ffn_fused_kernel(const __grid_constant__ FusedLaunch a) {
   __shared__ float red[2][WARPS][2 * NT * 4][32];  // two reduction buffers, used alternately
   __shared__ typename GroupOf<Q4>::type sg[Q4 ? kMaxFusedGroupsQ4 : kMaxFusedGroups];
   __shared__ int meta[3];
+  let_successor_start();
   build_chunk_table(a, sg, meta);
   __syncthreads();
   const int n = meta[0], tiles_gu = meta[1], tiles_dn = meta[2];
