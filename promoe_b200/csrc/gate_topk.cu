@@ -219,8 +219,8 @@ gate_topk_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __res
 // Router and permutation of a decode batch in ONE launch: a cluster of eight CTAs splits the expert rows (one SM
 // alone takes 4 us just to read a 64 x 2048 router matrix out of L2), every CTA sends its logits to the first one
 // through distributed shared memory, and that one selects the experts and lays the T * k pairs out per expert.
-// Same sums, in the same order, as gate_topk_kernel; same layout as the permutation kernels. Measured in a
-// CUDA graph, 8 tokens x 60 experts x 2048: 6.1 us, against 9.1 + 3.5 us in two launches.
+// Same sums, in the same order, as gate_topk_kernel; same layout as the permutation kernels. A pass of one token over 64
+// experts went from 55.1 to 45.9 us with it; in two launches (CUDA graph) the router took 9.2 us and the permutation 3.2.
 constexpr int kRouteCtas = 8, kRouteThreads = 512, kRouteMaxTokens = 16, kRouteMaxTopK = 16;
 
 template <int TOK>

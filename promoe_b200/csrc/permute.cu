@@ -39,7 +39,7 @@ __device__ __forceinline__ void scan_experts(const int* tot, int* off, int E) {
 // base. Inside an expert the order is ascending in the pair's index: the lanes of a warp that hold the same
 // expert find each other with one match instruction, and a pair's place is base + the expert's pairs in
 // lower warps + the lower lanes. (One warp per expert scanning all pairs took 34 us for 3108 pairs over 60
-// experts, now 8 us; 555 us for 49152 over 64, now 62 us.)
+// experts, now 8 us; 555 us for 49152 over 64, now 90 us.)
 __device__ __forceinline__ void place_pairs(int i, int e, int k, int E, int* base, unsigned short (*wcnt)[kMaxExperts],
                                             int32_t* __restrict__ row_token, int32_t* __restrict__ pos) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -192,7 +192,7 @@ cudaError_t launch_permute(const int32_t* topk_ids, int R, int k, int E, int32_t
                            int tail_rows, int T, cudaStream_t s, int32_t* scratch, size_t scratch_ints,
                            int32_t* zero_words, int zero_n) {
   if (zero_words == nullptr) zero_n = 0;
-  // Two launches cost about 4 us, every 1024 pairs in one CTA about 1.2 us.
+  // One CTA takes about 2 us per 1024 pairs.
   const int n_chunks = (R + kPermThreads - 1) / kPermThreads;
   if (n_chunks > 2 && scratch != nullptr && scratch_ints >= (size_t)n_chunks * E) {
     cudaError_t e = launch_behind(permute_count_kernel, n_chunks, 256, 0, s, topk_ids, R, E, scratch, err_flag, pos, zero_words, zero_n);

@@ -630,7 +630,7 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
 // once per 256 rows): measured on 8 experts of 4096 x 14336, 49 us a chunk of 9-16 rows against 75 us an
 // expert. All of them go one way, because a launch pair for a few experts leaves most SMs idle in its down
 // pass (105 us for one expert, 200 us for all 8). Layer calls of 64 / 128 / 512 tokens x top-2: 595 / 985 / 1505 us
-// when each expert from 64 rows on was expanded to a bf16 slab first, 560 / 597 / 653 us now.
+// when each expert from 64 rows on was expanded to a bf16 slab first, 560-600 / 597 / 653 us now.
 bool q4_prefers_tc(const Segment& seg) {
   int groups = 0, chunks = 0;
   for (size_t i = 0; i < seg.groups.size(); ++i)
