@@ -132,13 +132,13 @@ __device__ __forceinline__ void build_table(TcShared& sh, const TcGroup* __restr
     TcGroup g;
     if (groups != nullptr) {
       g = groups[i];
-    } else {  // group 0 is the shared expert where there is one, then the experts in order, absent ones with no rows
+    } else {  // group 0 is the shared expert where there is one, then the experts in order, those left out with no rows
       const int e = i - (plan.shared_inter > 0 ? 1 : 0);
       if (e < 0) {
         g = TcGroup{plan.n_routed_rows, plan.tokens, plan.shared_inter, -1};
       } else {
-        const int slot = plan.slot_table[e];
-        g = TcGroup{plan.offsets[e], slot >= 0 ? plan.counts[e] : 0, plan.inter, plan.first_line + slot};
+        const int slot = plan.slot_table[e], rows = plan.counts[e];
+        g = TcGroup{plan.offsets[e], slot >= 0 && rows >= plan.min_rows ? rows : 0, plan.inter, plan.first_line + slot};
       }
     }
     TcSlot t;

@@ -59,6 +59,10 @@ constexpr int kSplitTileDn = 32;    // or 32 down rows
 // (2048 x 1408, shared 5632) 224 -> 204, 254 -> 228, 279 -> 247, 314 -> 269 us. With the line at 0, 32 tokens x
 // top-6 over 64 experts lose: 155 us in chunks against 177 us.
 constexpr int kSplitChunkedMaxRows = 32;
+// Fewest rows of a uint4 group that may run on the tensor cores. They take weights rounded to bf16 after
+// dequantisation; the split-K tiles multiply the nibbles exactly and apply scale and zero to float32 sums
+// (error of a layer call against 64 bits 2.4e-3 instead of 3.7e-3), and keep every group below this line.
+constexpr int kQ4TcMinRows = 64;
 
 // Launches of one layer call follow each other closely: with launch_behind a kernel may be scheduled while its
 // predecessor in the stream drains (programmatic dependent launch). It has to call wait_for_predecessor before it
@@ -162,6 +166,7 @@ struct ResidentArgs {
   int32_t num_expert, inter, shared_inter, shared_slice;
   int32_t tokens, n_routed_rows;
   int32_t chunk_rows, quant4;
+  int32_t max_rows;  // experts with more rows are left to the host's plan
 };
 // Rows per chunk of such a launch when an expert may have up to row_bound rows. bf16: the kernel variant for 8 rows
 // or the one for 16. uint4: chunks of 8, the unpacking limits that kernel and its 16-row variant takes 1.6
@@ -169,7 +174,8 @@ struct ResidentArgs {
 inline int resident_chunk_rows(int row_bound, int quant4) { return quant4 || row_bound <= 8 ? 8 : 16; }
 // Most chunks such a launch can have.
 inline int resident_max_chunks(const ResidentArgs& a, int row_bound) {
-  const int per = (row_bound + a.chunk_rows - 1) / a.chunk_rows;
+  const int most = row_bound < a.max_rows ? row_bound : a.max_rows;
+  const int per = (most + a.chunk_rows - 1) / a.chunk_rows;
   const int routed = a.n_routed_rows / a.chunk_rows + a.num_expert;
   const int slices = a.shared_inter > 0 ? (a.shared_inter + a.shared_slice - 1) / a.shared_slice : 0;
   return (routed < per * a.num_expert ? routed : per * a.num_expert) + slices * ((a.tokens + a.chunk_rows - 1) / a.chunk_rows);
@@ -233,11 +239,11 @@ struct TcGroup {
   int32_t line;  // global cache line of the expert, -1 = the shared expert
 };
 // The groups of a launch pair as the device knows them behind the router: the shared expert (if any) and every
-// activated expert the layer's slot table shows resident.
+// activated expert the layer's slot table shows resident. Experts with fewer than min_rows rows are left to the host's plan.
 struct TcPlan {
   const int32_t *counts, *offsets, *slot_table;
   int32_t num_expert, first_line;  // first_line: global cache line of slot 0
-  int32_t inter, shared_inter, tokens, n_routed_rows;
+  int32_t inter, shared_inter, tokens, n_routed_rows, min_rows;
 };
 constexpr int kTcMaxN = 256;       // token rows per tile
 constexpr int kMaxTcGroups = 264;  // groups of one launch pair (every expert and the shared one)

@@ -625,22 +625,6 @@ int flush_segment_tc(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const _
   return PM_OK;
 }
 
-// Whether the uint4 experts of a segment go to the tensor cores. The split-K kernel's time follows the 16-row
-// chunks (it unpacks the weights once per chunk), the tensor-core kernel's the experts (it expands them
-// once per 256 rows): measured on 8 experts of 4096 x 14336, 49 us a chunk of 9-16 rows against 75 us an
-// expert. All of them go one way, because a launch pair for a few experts leaves most SMs idle in its down
-// pass (105 us for one expert, 200 us for all 8). Layer calls of 64 / 128 / 512 tokens x top-2: 595 / 985 / 1505 us
-// when each expert from 64 rows on was expanded to a bf16 slab first, 560-600 / 597 / 653 us now.
-bool q4_prefers_tc(const Segment& seg) {
-  int groups = 0, chunks = 0;
-  for (size_t i = 0; i < seg.groups.size(); ++i)
-    if (seg.group_line[i] >= 0 && seg.groups[i].row_count > 0) {
-      ++groups;
-      chunks += (seg.groups[i].row_count + kSplitMaxRows - 1) / kSplitMaxRows;
-    }
-  return 2 * chunks > 3 * groups;
-}
-
 // Groups on the split-K / staged kernels: plan them, upload the plan, launch. All groups are of one kind
 // (quant4, or bf16).
 int flush_groups_split(pm_ctx* c, const std::vector<pm_ffn_group>& groups, bool quant4, bool tc_ok, const pm_layer_weights& w,
@@ -703,10 +687,9 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
   }
   // A segment with groups of many rows goes to the tensor cores; otherwise the split-K tiles stream the
   // weights faster when there are only a few rows to use them for. There a group runs as chunks of 16 rows:
-  // its weights are read once from HBM and again from L2 for the later chunks.
+  // its weights are read once from HBM and again from L2 for the later chunks. uint4 groups go by their own rows.
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
   const bool tc_shared_ok = tc_shared_usable(w);
-  const bool q4_tc = w.quant4 && tc_ok && q4_prefers_tc(*seg);
   bool bf16_tc = false;
   for (const pm_ffn_group& g : seg->groups) bf16_tc = bf16_tc || g.row_count > kSplitChunkedMaxRows;
   Segment big, big_shared;  // the shared expert of a uint4 layer is bf16: it goes in a launch of its own
@@ -714,7 +697,8 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
     size_t keep = 0;
     for (size_t i = 0; i < seg->groups.size(); ++i) {
       const bool shared = seg->group_line[i] < 0;
-      const bool many = !w.quant4 ? bf16_tc : shared ? seg->groups[i].row_count > kSplitChunkedMaxRows : q4_tc;
+      const int rows = seg->groups[i].row_count;
+      const bool many = !w.quant4 ? bf16_tc : shared ? rows > kSplitChunkedMaxRows : rows >= kQ4TcMinRows;
       if (many && (!shared || tc_shared_ok)) {
         Segment& to = shared && w.quant4 ? big_shared : big;
         to.groups.push_back(seg->groups[i]);
@@ -865,10 +849,10 @@ enum class DevicePlan { kNone, kSplit, kTc };
 // Which kernel it uses has to follow from the sizes alone:
 //  bf16   up to 32 rows per expert the split-K kernel, as flush_segment chooses; above, a shared expert (T rows) would
 //         take the call to the tensor cores, and so do 16 rows per expert on average without one
-//  uint4  up to 8 rows per expert on average split-K chunks, from 24 on the tensor cores (q4_prefers_tc's line lies
-//         at about 16)
+//  uint4  up to 8 rows per expert on average split-K chunks, from 64 on the tensor cores
 // and what is in between waits for the counts. A bf16 shared expert beside uint4 experts does too, and so do
-// caller-routed rows that could be many: most of those may be padding.
+// caller-routed rows that could be many: most of those may be padding. A uint4 launch takes the experts on its side
+// of kQ4TcMinRows, the others follow from the host's plan.
 DevicePlan choose_device_plan(pm_ctx* c, int layer, const pm_layer_weights& w, bool has_shared, bool sliced, bool routed,
                               int T, int R, int row_bound, ResidentArgs* a) {
   if (!c->device_plan || (w.quant4 && has_shared)) return DevicePlan::kNone;
@@ -900,7 +884,8 @@ DevicePlan choose_device_plan(pm_ctx* c, int layer, const pm_layer_weights& w, b
   a->chunk_rows = resident_chunk_rows(row_bound, w.quant4);
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w) && (!has_shared || tc_shared_usable(w));
   const bool split = w.quant4 ? R <= 8 * E || !tc_ok : row_bound <= kSplitChunkedMaxRows;
-  const bool tc = tc_ok && !routed && (w.quant4 ? R >= 24 * E : row_bound > kSplitChunkedMaxRows && (has_shared || R >= 16 * E));
+  a->max_rows = w.quant4 && tc_ok ? kQ4TcMinRows - 1 : R;
+  const bool tc = tc_ok && !routed && (w.quant4 ? R >= kQ4TcMinRows * E : row_bound > kSplitChunkedMaxRows && (has_shared || R >= 16 * E));
   if (split && resident_ffn_available(a->chunk_rows, w.quant4) &&
       resident_max_chunks(*a, row_bound) <= (w.quant4 ? kMaxFusedGroupsQ4 : kMaxFusedGroups))
     return DevicePlan::kSplit;
@@ -1079,7 +1064,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
       TcLaunch a = tc_launch_args(c, w, w.quant4 != 0);
       a.groups_dev = nullptr;
       a.plan = TcPlan{res.counts, res.offsets, res.slot_table, E, c->eng->pools()[c->eng->pool_index(layer)].base,
-                      w.inter, res.shared_inter, T, R};
+                      w.inter, res.shared_inter, T, R, w.quant4 ? kQ4TcMinRows : 0};
       a.n_groups = E + (has_shared ? 1 : 0);
       a.max_rows = row_bound;
       a.tiles_gu = a.tiles_dn = 1 << 20;  // only known on the device: full grids
@@ -1135,6 +1120,9 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   if (can_evict)
     for (int e = 0; e < E; ++e)
       if (resident_line[e] >= 0 && counts[e] == 0) c->line_read[resident_line[e]] = read_before[e];
+  if (spec)  // experts the device-planned launch left out
+    for (int e = 0; e < E; ++e)
+      if (plan == DevicePlan::kTc ? w.quant4 && counts[e] < kQ4TcMinRows : counts[e] > res.max_rows) resident_line[e] = -1;
   if (keep) {
     c->last_ids[layer].assign(st.ids, st.ids + R);
     c->last_w[layer].assign(st.w, st.w + R);

@@ -883,7 +883,7 @@ __device__ __forceinline__ void build_chunk_table(const FusedLaunch& a, G* sg, i
         slot = r.slot_table[e];
         off = r.offsets[e];
       }
-      const int n = slot >= 0 ? (cnt + r.chunk_rows - 1) / r.chunk_rows : 0;
+      const int n = slot >= 0 && cnt <= r.max_rows ? (cnt + r.chunk_rows - 1) / r.chunk_rows : 0;
       int incl = n;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {

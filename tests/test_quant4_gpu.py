@@ -206,3 +206,74 @@ def test_gptq_checkpoint_layout_through_inject_model(lib):
             got = ys[l].float().cpu().numpy().reshape(5, H)
             np.testing.assert_allclose(got, ref, rtol=RTOL_Q4, atol=RTOL_Q4 * np.abs(ref).max() * 0.25)
     assert mngr.metas.cache.stats()["precise_miss"] > 0
+
+
+def q4_cache(model_experts, rng, H, I, k, gate_w=None, gate_bias=None, norm=False):
+    """A one-layer cache of uint4 experts, all resident; returns it and the dequantised matrices."""
+    from promoe_b200.engine import ExpertCache
+    E = model_experts
+    cache = ExpertCache(1, E, num_expert_per_token=k, cache_rate=1.0, num_predict_expert_per_layer=0)
+    cache.set_param_list(["w1.qweight", "w1.scale_zero", "w3.qweight", "w3.scale_zero", "w2.qweight", "w2.scale_zero"])
+    deq = []
+    for e in range(E):
+        _, q, raw = q4_expert(rng, H, I)
+        deq.append(tuple(q))
+        cache.register_expert(0, e, raw)
+    cache.pin_all()
+    cache.build_slab()
+    if gate_w is None:
+        cache.set_layer_weights(0, None, I, 1, False, 1.0, hidden=H, quant4=True)
+    else:
+        cache.set_layer_weights(0, dev_bf16(gate_w), I, k, norm, gate_bias=dev(gate_bias), quant4=True)
+    return cache, deq
+
+
+# The split-K tiles multiply the nibbles exactly; against an oracle that rounds the intermediate row as they do,
+# what is left is float32 summation and a few flipped roundings of that row, a few 1e-4. Weights rounded to bf16
+# (relative error 2^-9 at most, 2^-9 / sqrt(3) on average) would put 1e-3 per matrix on it, 2e-3 in all.
+EXACT_Q4 = 8e-4
+
+
+@pytest.mark.parametrize("counts,expanded", [([63, 17, 0, 40, 1], 0), ([64, 63, 25], 1), ([8, 200, 33, 64], 2)])
+def test_q4_weights_stay_exact_below_64_rows(lib, counts, expanded):
+    H, I, E = 512, 384, len(counts)
+    rng = np.random.default_rng(11 + E)
+    cache, deq = q4_cache(E, rng, H, I, 1)
+    ids = np.repeat(np.arange(E, dtype=np.int32), counts)
+    rng.shuffle(ids)
+    x = om.bf16_round(rng.standard_normal((len(ids), H)).astype(np.float32))
+    xd, idd = dev_bf16(x), dev(ids)
+    out = torch.full((len(ids), H), float("nan"), dtype=torch.float32, device="cuda")
+    _lib.call("pm_moe_forward_routed", cache.handle, 0, ptr(xd), len(ids), ptr(idd), ptr(out), 0, None, None, 0, 0, 0, 0, None)
+    torch.cuda.synchronize()
+    assert int(cache.get("q4_expanded")) == expanded and cache.get("tc_error") == "0"
+    cache.close()
+    got = out.cpu().numpy()
+    for e, n in enumerate(counts):
+        if n:
+            ref = om.swiglu_mlp(x[ids == e], *deq[e], round_h_bf16=True)
+            err = np.linalg.norm(got[ids == e] - ref) / np.linalg.norm(ref)
+            assert err < (EXACT_Q4 if n < 64 else 5e-3), (e, n, err)
+
+
+# layer calls, whose launch may be planned on the device: every expert below the line (average 30 rows); one expert of
+# many rows among small ones (average 2 and 8 rows: chunks of 8); prompts with experts on both sides of the line
+@pytest.mark.parametrize("E,k,T,popular,lift", [(4, 2, 60, 0, 0.0), (48, 1, 100, 1, 1.1), (12, 1, 90, 1, 0.95),
+                                                (4, 1, 300, 1, 0.5), (6, 2, 250, 2, 0.7)])
+def test_q4_layer_call_expands_only_experts_of_64_rows(lib, E, k, T, popular, lift):
+    H, I = 256, 128
+    rng = np.random.default_rng(5 * E + T)
+    gate_w = bf16_weights(rng, (E, H), 0.02)
+    bias = np.zeros(E, np.float32)
+    bias[:popular] = lift
+    cache, deq = q4_cache(E, rng, H, I, k, gate_w, bias)
+    cache.set("keep_routing", 1)
+    x = om.bf16_round(rng.standard_normal((T, H)).astype(np.float32))
+    y = cache.forward(0, dev_bf16(x)).float().cpu().numpy()
+    ids, _ = cache.last_routing(0, T, k)
+    counts = np.bincount(ids.ravel(), minlength=E)
+    assert (counts.max() >= 64) == (popular > 0) and (counts < 64).any()
+    assert int(cache.get("q4_expanded")) == int((counts >= 64).sum()) and cache.get("tc_error") == "0"
+    cache.close()
+    ref, _, _ = om.moe_block_forward(x, gate_w, deq, k, False, gate_bias=bias, round_h_bf16=True)
+    np.testing.assert_allclose(y, ref, rtol=RTOL_Q4, atol=RTOL_Q4 * np.abs(ref).max() * 0.25)
