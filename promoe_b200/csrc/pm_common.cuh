@@ -51,8 +51,8 @@ constexpr int kMaxChunkRows = 64;   // token rows per chunk (8 MMA n-tiles)
 constexpr int kSplitMaxRows = 16;   // launches whose chunks all fit use the split-K decode kernel,
 constexpr int kSplitTileGu = 16;    // whose tiles are 16 gate+up rows
 constexpr int kSplitTileDn = 32;    // or 32 down rows
-// Most rows of a bf16 group for which its segment stays on the split-K kernel (as chunks of 16 rows). One group
-// above it takes all groups of the segment to the tensor cores, whose launch pair streams the weights of
+// Most rows of a bf16 group for which its layer call stays on the split-K kernel (as chunks of 16 rows). One group
+// above it takes all groups of the call to the tensor cores, whose launch pair streams the weights of
 // every group once; two kinds of launches after one another each leave SMs idle at their ends. Measured
 // (FFN of one layer, mixed launches with the same line -> one kind): 64 tokens x top-8, experts of 1-40 rows
 // (hidden 3584, inter 2560, shared 20480) 773 -> 716 us; 100 / 200 / 400 / 777 tokens x top-4 over 60 experts

@@ -518,6 +518,7 @@ struct PendingForward {
   bool active = false;
   int layer = 0, T = 0, R = 0, n_shared = 0, k = 1, H = 0;
   bool spec = false, is_routed = false;
+  bool bf16_tc = false;  // the bf16 groups of this call run on the tensor cores
   pm_layer_weights w{};
   const __nv_bfloat16* x = nullptr;
   void* yv = nullptr;
@@ -675,7 +676,7 @@ int flush_groups_split(pm_ctx* c, const std::vector<pm_ffn_group>& groups, bool 
   return PM_OK;
 }
 
-int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows,
+int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv_bfloat16* x, int n_rows, bool bf16_tc,
                   size_t* desc_used, cudaStream_t s) {
   if (seg->empty()) return PM_OK;
   for (int line : seg->waits) {
@@ -685,13 +686,10 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
       c->line_waiter[line] = s;
     }
   }
-  // A segment with groups of many rows goes to the tensor cores; otherwise the split-K tiles stream the
-  // weights faster when there are only a few rows to use them for. There a group runs as chunks of 16 rows:
-  // its weights are read once from HBM and again from L2 for the later chunks. uint4 groups go by their own rows.
+  // bf16 groups go where bf16_call_on_tc sends the call, uint4 groups by their own rows. On the split-K tiles a group
+  // runs as chunks of 16 rows: its weights are read once from HBM and again from L2 for the later chunks.
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
   const bool tc_shared_ok = tc_shared_usable(w);
-  bool bf16_tc = false;
-  for (const pm_ffn_group& g : seg->groups) bf16_tc = bf16_tc || g.row_count > kSplitChunkedMaxRows;
   Segment big, big_shared;  // the shared expert of a uint4 layer is bf16: it goes in a launch of its own
   if (tc_ok) {
     size_t keep = 0;
@@ -785,7 +783,7 @@ int run_actions(pm_ctx* c, PendingForward& p, bool collect, bool* stopped) {
           *stopped = true;
           return PM_OK;
         }
-        int rc = flush_segment(c, &p.seg, p.w, p.x, n_rows, &p.desc_used, s);
+        int rc = flush_segment(c, &p.seg, p.w, p.x, n_rows, p.bf16_tc, &p.desc_used, s);
         if (rc != PM_OK) return rc;
         p.seg_waits_for_pooled = false;
       }
@@ -806,7 +804,7 @@ int run_actions(pm_ctx* c, PendingForward& p, bool collect, bool* stopped) {
       const bool must_wait = c->line_pending[a.line] || (c->line_waiter[a.line] != nullptr && c->line_waiter[a.line] != s);
       if (must_wait && p.seg.waits.empty() && !p.seg.empty()) {
         // let everything that is already resident run while the copies are in flight
-        int rc = flush_segment(c, &p.seg, p.w, p.x, n_rows, &p.desc_used, s);
+        int rc = flush_segment(c, &p.seg, p.w, p.x, n_rows, p.bf16_tc, &p.desc_used, s);
         if (rc != PM_OK) return rc;
       }
       p.seg.groups.push_back(group_of_line(c, p, a.expert, a.line));
@@ -822,7 +820,7 @@ int run_actions(pm_ctx* c, PendingForward& p, bool collect, bool* stopped) {
     *stopped = true;
     return PM_OK;
   }
-  return flush_segment(c, &p.seg, p.w, p.x, n_rows, &p.desc_used, s);
+  return flush_segment(c, &p.seg, p.w, p.x, n_rows, p.bf16_tc, &p.desc_used, s);
 }
 
 int finish_forward(pm_ctx* c, PendingForward& p) {
@@ -842,13 +840,22 @@ int finish_forward(pm_ctx* c, PendingForward& p) {
 
 namespace {
 
+// Whether the bf16 groups of a layer call run on the tensor cores: with a group of more than kSplitChunkedMaxRows
+// rows (a shared expert has T) all of them do, without a shared expert also from 16 rows per expert on average. A rule
+// on the call, not on a launch: the two kernels add in different orders, and which experts share a launch depends on
+// what the cache held. max_rows: rows of the largest expert, 0 while only the sizes are known.
+bool bf16_call_on_tc(bool has_shared, bool routed, int R, int E, int row_bound, int max_rows) {
+  if (max_rows > kSplitChunkedMaxRows) return true;
+  return !routed && row_bound > kSplitChunkedMaxRows && (has_shared || R >= 16 * E);
+}
+
 // The launch for the shared expert and the experts already resident, enqueued behind the router without waiting for
 // the host to read the row counts (25 to 35 us of an idle GPU per layer call otherwise).
 enum class DevicePlan { kNone, kSplit, kTc };
 
 // Which kernel it uses has to follow from the sizes alone:
-//  bf16   up to 32 rows per expert the split-K kernel, as flush_segment chooses; above, a shared expert (T rows) would
-//         take the call to the tensor cores, and so do 16 rows per expert on average without one
+//  bf16   up to 32 rows per expert the split-K kernel; above, the tensor cores where bf16_call_on_tc follows from
+//         the sizes
 //  uint4  up to 8 rows per expert on average split-K chunks, from 64 on the tensor cores
 // and what is in between waits for the counts. A bf16 shared expert beside uint4 experts does too, and so do
 // caller-routed rows that could be many: most of those may be padding. A uint4 launch takes the experts on its side
@@ -885,7 +892,7 @@ DevicePlan choose_device_plan(pm_ctx* c, int layer, const pm_layer_weights& w, b
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w) && (!has_shared || tc_shared_usable(w));
   const bool split = w.quant4 ? R <= 8 * E || !tc_ok : row_bound <= kSplitChunkedMaxRows;
   a->max_rows = w.quant4 && tc_ok ? kQ4TcMinRows - 1 : R;
-  const bool tc = tc_ok && !routed && (w.quant4 ? R >= kQ4TcMinRows * E : row_bound > kSplitChunkedMaxRows && (has_shared || R >= 16 * E));
+  const bool tc = tc_ok && (w.quant4 ? !routed && R >= kQ4TcMinRows * E : bf16_call_on_tc(has_shared, routed, R, E, row_bound, 0));
   if (split && resident_ffn_available(a->chunk_rows, w.quant4) &&
       resident_max_chunks(*a, row_bound) <= (w.quant4 ? kMaxFusedGroupsQ4 : kMaxFusedGroups))
     return DevicePlan::kSplit;
@@ -1178,6 +1185,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   p = PendingForward();
   p.layer = layer; p.T = T; p.R = R; p.n_shared = n_shared; p.k = k; p.H = H;
   p.spec = spec; p.is_routed = routed != nullptr;
+  p.bf16_tc = bf16_call_on_tc(has_shared, routed != nullptr, R, E, row_bound, *std::max_element(counts, counts + E));
   p.w = w; p.x = x; p.yv = yv; p.rows_out = routed ? routed->rows_out : nullptr; p.s = s;
   p.acts = std::move(acts);
   p.ids = ids;

@@ -3,12 +3,13 @@ read the row counts): experts with more rows than one chunk, absent experts, bot
 oracle; cache log exact."""
 import numpy as np
 import pytest
+import torch
 
 from oracle import quant4 as oq
 from oracle import srs_policy as sp
 from promoe_b200 import quant4 as pq
 from promoe_b200.engine import ExpertCache
-from tests.helpers import TinyModel, dev_bf16
+from tests.helpers import TinyModel, dev, dev_bf16
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +54,38 @@ def test_uint4_batches(lib, T, rate):
     cache.build_slab()
     cache.set_layer_weights(0, dev_bf16(model.gate_w[0]), model.I, 2, True, quant4=True)
     check(model, cache, T, rate, 6, 3e-2)
+
+
+def q4_model_cache(model, rate):
+    """A cache of the model's experts as uint4 (packed once and kept on the model)."""
+    if not hasattr(model, "raw"):
+        model.raw = [[[t for w in model.experts[l][e] for t in pq.quantize_pack(w)] for e in range(model.E)]
+                     for l in range(model.L)]
+    cache = ExpertCache(model.L, model.E, num_expert_per_token=model.k, cache_rate=rate, num_predict_expert_per_layer=0)
+    cache.set_param_list(["w1.qweight", "w1.scale_zero", "w3.qweight", "w3.scale_zero", "w2.qweight", "w2.scale_zero"])
+    for l in range(model.L):
+        for e in range(model.E):
+            cache.register_expert(l, e, model.raw[l][e])
+    cache.pin_all()
+    cache.build_slab()
+    for l in range(model.L):
+        cache.set_layer_weights(l, dev_bf16(model.gate_w[l]), model.I, model.k, model.norm_topk,
+                                gate_bias=dev(model.gate_bias[l]), quant4=True)
+    return cache
+
+
+# experts that are found, that have to be copied, and that are copied one after another into too few lines: the launches
+# differ, the numbers may not (T on either side of every line between two kernels)
+@pytest.mark.parametrize("T", [20, 33, 48, 70, 200])
+@pytest.mark.parametrize("kind", ["shared", "plain", "uint4"])
+def test_outputs_do_not_depend_on_what_the_cache_held(lib, kind, T):
+    model = TinyModel(seed=3 * T, L=1, E=8, H=1024, I=512, k=2, shared_I=512 if kind == "shared" else 0)
+    xd = dev_bf16(model.hidden_stream(T, 1)[0])
+    ys = []
+    for rate in (1.0, 0.5, 0.25):
+        cache = (q4_model_cache(model, rate) if kind == "uint4"
+                 else model.make_cache(cache_rate=rate, num_predict_expert_per_layer=0))
+        ys += [cache.forward(0, xd).clone() for _ in range(3)]
+        assert cache.get("tc_error") == "0"
+        cache.close()
+    assert all(torch.equal(ys[0], y) for y in ys[1:])
