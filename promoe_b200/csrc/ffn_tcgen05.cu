@@ -532,7 +532,7 @@ prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ 
             const uint32_t other = __shfl_xor_sync(0xffffffffu, upper ? v[c] : v[c + 1], 16);
             const uint32_t lo = upper ? other : v[c], hi = upper ? v[c + 1] : other;
             const float gv = __uint_as_float(up_first ? hi : lo), uv = __uint_as_float(up_first ? lo : hi);
-            const float h = __fdividef(gv, 1.f + __expf(-gv)) * uv;
+            const float h = gv / (1.f + __expf(-gv)) * uv;  // a full division: __fdividef gives 0 for denominators above 2^126
             if (c < left) dst[(size_t)c * ld_h] = __float2bfloat16_rn(h);
           }
         } else {

@@ -138,3 +138,34 @@ def test_uint4_layer_with_bf16_shared_expert(lib):
         ref, _, _ = model.oracle_forward(0, x)
         assert np.linalg.norm(y - ref) / np.linalg.norm(ref) < 8e-3
     cache.close()
+
+
+@pytest.mark.parametrize("rows", [40, 20])  # the tensor cores; the split-K tiles
+def test_silu_of_large_negative_gates(lib, rows):
+    """The quotient -g / (1 + e^g) just above g = 87 is a normal float32 (some 1e-36) that a large up value brings
+    back into range; an approximate division returns 0 for denominators above 2^126."""
+    H = I = 64
+    rng = np.random.default_rng(rows)
+    wg, wu = np.zeros((I, H), np.float32), np.zeros((I, H), np.float32)
+    wg[:, 0] = rng.choice([-87.5, -88.0, -88.5, -3.0, 2.0], size=I)
+    wu[:, 0] = np.where(wg[:, 0] < -87, np.float32(2.0) ** 100, np.float32(2.0) ** -20)
+    wd = bf16_weights(rng, (H, I))
+    cache = ExpertCache(1, 1, num_expert_per_token=1, cache_rate=1.0, num_predict_expert_per_layer=0)
+    cache.set_param_list(["gate_proj.weight", "up_proj.weight", "down_proj.weight"])
+    cache.register_expert(0, 0, [om.to_bf16_bits(m) for m in (wg, wu, wd)])
+    cache.pin_all()
+    cache.build_slab()
+    cache.set_layer_weights(0, None, I, 1, False, 1.0, hidden=H)
+    x = np.zeros((rows, H), np.float32)
+    x[:, 0] = 1.0
+    xd, idd = dev_bf16(x), torch.zeros(rows, dtype=torch.int32, device="cuda")
+    out = torch.empty((rows, H), dtype=torch.float32, device="cuda")
+    _lib.call("pm_moe_forward_routed", cache.handle, 0, xd.data_ptr(), rows, idd.data_ptr(), out.data_ptr(), 0, None, None,
+              0, 0, 0, 0, None)
+    torch.cuda.synchronize()
+    assert (int(cache.get("tc_launches")) > 0) == (rows > 32)
+    cache.close()
+    ref = om.swiglu_mlp(x, wg, wu, wd, round_h_bf16=True)
+    assert np.abs(ref).max() > 1e-8
+    # __expf is off by 2 ulp + |x| * 2^-22 in its exponent (2e-5 here), the row is rounded to bf16
+    np.testing.assert_allclose(out.cpu().numpy(), ref, rtol=2e-2, atol=2e-2 * np.abs(ref).max() * 0.25)
