@@ -523,10 +523,17 @@ __device__ __forceinline__ void tile_issue_a(const TileCtx<NT>& t, int s0, uint4
   }
 }
 
+// Whether a uint4 tile fetches its token values a step ahead of their use: out of L1 / L2 they take 300 cycles and
+// more (8 experts of 4096 x 14336, 16 tokens in chunks of 8 rows: 215 us when they were loaded where they are
+// used, 200 us). Not for 16-row chunks, whose 32 registers more are spilled (776 bytes instead of 504): layer calls of
+// 33 / 64 tokens x top-2 over the same experts 463 / 677 us with it, 372 / 531 without.
+template <int NT>
+constexpr bool kQ4Ahead = NT == 1;
+
 template <int NT, int DEPTH, bool COHERENT_B, bool Q4, int FIRST = 0, int COUNT = DEPTH>
 __device__ __forceinline__ void tile_issue_b(const TileCtx<NT>& t, int s0, uint4 (&b)[DEPTH][NT], uint4 (&bq)[NT][4]) {
-  if constexpr (Q4) {  // the first step's token values; tile_compute_q4 fetches each later step's one step ahead
-    if (FIRST == 0 && s0 < t.s_end) {
+  if constexpr (Q4) {  // the first step's token values (see kQ4Ahead); tile_compute_q4 fetches the later steps'
+    if (kQ4Ahead<NT> && FIRST == 0 && s0 < t.s_end) {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -587,11 +594,13 @@ __device__ __forceinline__ void tile_compute_q4(const TileCtx<NT>& t, int s0, co
         uint4 bv[NT];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-          bv[nt] = bq[nt][v];
-          // the next step's token values, a whole step ahead of their use: out of L1 / L2 they take 300 cycles and
-          // more (8 experts of 4096 x 14336, 16 tokens: 215 us when they were loaded where they are used, 200 us)
-          if (s0 + d + 1 < t.s_end)
-            bq[nt][v] = load_b<COHERENT_B>(t.b_ptr[nt] + (size_t)(s0 + d + 1) * 256 + v * 16);
+          if constexpr (kQ4Ahead<NT>) {
+            bv[nt] = bq[nt][v];
+            if (s0 + d + 1 < t.s_end)
+              bq[nt][v] = load_b<COHERENT_B>(t.b_ptr[nt] + (size_t)(s0 + d + 1) * 256 + v * 16);
+          } else {
+            bv[nt] = load_b<COHERENT_B>(t.b_ptr[nt] + (size_t)(s0 + d) * 256 + v * 16);
+          }
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {  // nibble pairs {0,1} go with b.x, b.y; pairs {2,3} with b.z, b.w
