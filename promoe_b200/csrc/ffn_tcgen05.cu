@@ -295,7 +295,11 @@ prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ 
         const uint32_t bar = map_to_rank(smem_u32(&sh.full[at.slot]), 0);
         unsigned char* dst = stages + (size_t)at.slot * ring.stage_bytes;
         if (!Q4) {
-          if (GATEUP) tma_load_5d(dst, map_w, bar, kt * 64, 0, 0, t.m * 8 + (int)rank * 4, line);
+          if (GATEUP && shared_expert && maps.sh_split) {
+#pragma unroll 1
+            for (int b = 0; b < 8; ++b)  // 16 gate rows, the 16 up rows, the next 16 gate rows, ...
+              tma_load_2d(dst + b * 2048, b & 1 ? &maps.sh_up : &maps.sh_gu, bar, kt * 64, t.m * 128 + (int)rank * 64 + (b >> 1) * 16);
+          } else if (GATEUP) tma_load_5d(dst, map_w, bar, kt * 64, 0, 0, t.m * 8 + (int)rank * 4, line);
           else tma_load_3d(dst, map_w, bar, kt * 64, t.m * 256 + (int)rank * 128, line);
         }
         dst += kWBytes;

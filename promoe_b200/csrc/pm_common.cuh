@@ -229,10 +229,12 @@ cudaError_t launch_combine(const float* yexp, const int32_t* pos, const float* t
 // about as much as 16 KB of data). Weights: routed experts through maps over the whole slab whose last
 // coordinate is the cache line, the layer's shared expert through maps of its own. The gate/up maps
 // see both matrices as (k, row in block of 16, matrix, block, line), so that one box of 4 blocks brings
-// 64 gate and 64 up rows, alternating in blocks of 16; the matrix with the lower address comes first.
+// 64 gate and 64 up rows, alternating in blocks of 16; the matrix with the lower address comes first. The
+// matrices of a shared expert are the caller's and may lie further apart than a map's stride reaches: then sh_split is set,
+// sh_gu and sh_up are 2-D maps of one matrix each, and a box brings 16 rows.
 struct TcMaps {
-  CUtensorMap a_x[4], a_h[4], slab_gu, slab_down, sh_gu, sh_down;
-  int32_t slab_up_first, sh_up_first;
+  CUtensorMap a_x[4], a_h[4], slab_gu, slab_down, sh_gu, sh_up, sh_down;
+  int32_t slab_up_first, sh_up_first, sh_split;
 };
 struct TcGroup {
   int32_t row_start, row_count, inter;

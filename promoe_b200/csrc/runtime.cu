@@ -689,7 +689,6 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
   // bf16 groups go where bf16_call_on_tc sends the call, uint4 groups by their own rows. On the split-K tiles a group
   // runs as chunks of 16 rows: its weights are read once from HBM and again from L2 for the later chunks.
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
-  const bool tc_shared_ok = tc_shared_usable(w);
   Segment big, big_shared;  // the shared expert of a uint4 layer is bf16: it goes in a launch of its own
   if (tc_ok) {
     size_t keep = 0;
@@ -697,7 +696,7 @@ int flush_segment(pm_ctx* c, Segment* seg, const pm_layer_weights& w, const __nv
       const bool shared = seg->group_line[i] < 0;
       const int rows = seg->groups[i].row_count;
       const bool many = !w.quant4 ? bf16_tc : shared ? rows > kSplitChunkedMaxRows : rows >= kQ4TcMinRows;
-      if (many && (!shared || tc_shared_ok)) {
+      if (many) {
         Segment& to = shared && w.quant4 ? big_shared : big;
         to.groups.push_back(seg->groups[i]);
         to.group_line.push_back(seg->group_line[i]);
@@ -889,7 +888,7 @@ DevicePlan choose_device_plan(pm_ctx* c, int layer, const pm_layer_weights& w, b
   a->n_routed_rows = R;
   a->quant4 = w.quant4;
   a->chunk_rows = resident_chunk_rows(row_bound, w.quant4);
-  const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w) && (!has_shared || tc_shared_usable(w));
+  const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
   const bool split = w.quant4 ? R <= 8 * E || !tc_ok : row_bound <= kSplitChunkedMaxRows;
   a->max_rows = w.quant4 && tc_ok ? kQ4TcMinRows - 1 : R;
   const bool tc = tc_ok && (w.quant4 ? !routed && R >= kQ4TcMinRows * E : bf16_call_on_tc(has_shared, routed, R, E, row_bound, 0));

@@ -228,7 +228,6 @@ void rt_mark_dirty(pm_ctx* c, const std::vector<Action>& actions);
 int rt_profile_collect(pm_ctx* c);
 bool tc_prefill_usable(const pm_ctx* c, const pm_layer_weights& w);
 bool tc_prefill_usable_q4(const pm_ctx* c, const pm_layer_weights& w);
-bool tc_shared_usable(const pm_layer_weights& w);  // one tensor map can span the shared gate and up matrices
 int tc_build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m);
 void tc_tile_count(const TcGroup& g, int hidden, int* gu, int* dn);  // adds the group's tiles
 

@@ -74,6 +74,13 @@ int encode_down(CUtensorMap* map, const void* down, uint64_t hidden, uint64_t in
   return encode(map, down, 3, dims, strides, box, packed);
 }
 
+// Whether one map can span two matrices: its strides are positive and stay below 2^40 bytes. Allocators do place
+// tensors of a program further apart than that.
+bool one_map_spans(const void* a, const void* b) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b, apart = x > y ? x - y : y - x;
+  return apart > 0 && apart < ((uintptr_t)1 << 40);
+}
+
 }  // namespace
 
 bool tc_prefill_usable(const pm_ctx* c, const pm_layer_weights& w) {
@@ -85,13 +92,6 @@ bool tc_prefill_usable(const pm_ctx* c, const pm_layer_weights& w) {
 bool tc_prefill_usable_q4(const pm_ctx* c, const pm_layer_weights& w) {
   if (!c->tc_prefill || !w.quant4 || encode_fn() == nullptr) return false;
   return w.hidden % 128 == 0 && w.inter % 128 == 0 && w.shared_inter % 64 == 0;
-}
-
-// Strides of a tensor map stay below 2^40 bytes: matrices further apart (memory of different allocators)
-// leave the shared expert on the other kernels.
-bool tc_shared_usable(const pm_layer_weights& w) {
-  const uintptr_t g = (uintptr_t)w.shared_w_gate, u = (uintptr_t)w.shared_w_up;
-  return (g > u ? g - u : u - g) < ((uintptr_t)1 << 40);
 }
 
 // Maps of the token rows, of the slab of expert lines and of the layer's shared expert. uint4 layers: the
@@ -108,16 +108,24 @@ int tc_build_maps(pm_ctx* c, const pm_layer_weights& w, int rows_cap, TcMaps* m)
   if (rc != PM_OK) return rc;
   rc = encode_down(&m->slab_down, c->slab + c->param_offset[c->role_down], H, I, stride, lines, packed);
   if (rc != PM_OK) return rc;
-  if (Is > 0 && tc_shared_usable(w)) {  // one "line"; its stride is never used but has to be a valid one
-    rc = encode_gate_up(&m->sh_gu, &m->sh_up_first, (const unsigned char*)w.shared_w_gate, (const unsigned char*)w.shared_w_up, H,
-                        Is, H * 32, 1);
+  // never dereferenced where they stay as they are here: any valid map keeps the parameter well formed
+  m->sh_gu = m->sh_up = m->slab_gu;
+  m->sh_down = m->slab_down;
+  m->sh_up_first = m->sh_split = 0;
+  if (Is > 0) {
+    m->sh_split = !one_map_spans(w.shared_w_gate, w.shared_w_up);
+    if (m->sh_split) {
+      const cuuint64_t dims[2] = {H, Is}, strides[1] = {H * 2};
+      const cuuint32_t box[2] = {64, 16};
+      rc = encode(&m->sh_gu, w.shared_w_gate, 2, dims, strides, box);
+      if (rc == PM_OK) rc = encode(&m->sh_up, w.shared_w_up, 2, dims, strides, box);
+    } else {  // one "line"; its stride is never used but has to be a valid one
+      rc = encode_gate_up(&m->sh_gu, &m->sh_up_first, (const unsigned char*)w.shared_w_gate, (const unsigned char*)w.shared_w_up, H,
+                          Is, H * 32, 1);
+    }
     if (rc != PM_OK) return rc;
     rc = encode_down(&m->sh_down, w.shared_w_down, H, Is, Is * 2, 1);
     if (rc != PM_OK) return rc;
-  } else {  // never dereferenced: any valid map keeps the parameter well formed
-    m->sh_gu = m->slab_gu;
-    m->sh_down = m->slab_down;
-    m->sh_up_first = 0;
   }
   return PM_OK;
 }

@@ -169,3 +169,80 @@ def test_silu_of_large_negative_gates(lib, rows):
     assert np.abs(ref).max() > 1e-8
     # __expf is off by 2 ulp + |x| * 2^-22 in its exponent (2e-5 here), the row is rounded to bf16
     np.testing.assert_allclose(out.cpu().numpy(), ref, rtol=2e-2, atol=2e-2 * np.abs(ref).max() * 0.25)
+
+
+class FarPair:
+    """Two device buffers 2^41 bytes apart: one address range with memory mapped at its two ends."""
+
+    def __init__(self, nbytes):
+        from cuda.bindings import driver as cu
+        self.cu, dev_id = cu, torch.cuda.current_device()
+        torch.zeros(1, device="cuda")
+        prop = cu.CUmemAllocationProp()
+        prop.type = cu.CUmemAllocationType.CU_MEM_ALLOCATION_TYPE_PINNED
+        prop.location.type = cu.CUmemLocationType.CU_MEM_LOCATION_TYPE_DEVICE
+        prop.location.id = dev_id
+        gran = self.ok(cu.cuMemGetAllocationGranularity(prop, cu.CUmemAllocationGranularity_flags.CU_MEM_ALLOC_GRANULARITY_MINIMUM))
+        self.size = -(-nbytes // gran) * gran
+        self.total = (1 << 41) + self.size
+        self.base = int(self.ok(cu.cuMemAddressReserve(self.total, gran, 0, 0)))
+        acc = cu.CUmemAccessDesc()
+        acc.location = prop.location
+        acc.flags = cu.CUmemAccess_flags.CU_MEM_ACCESS_FLAGS_PROT_READWRITE
+        self.at, self.handles = [self.base, self.base + (1 << 41)], []
+        for a in self.at:
+            h = self.ok(cu.cuMemCreate(self.size, prop, 0))
+            self.ok(cu.cuMemMap(a, self.size, 0, h, 0))
+            self.ok(cu.cuMemSetAccess(a, self.size, [acc], 1))
+            self.handles.append(h)
+
+    def ok(self, r):
+        assert int(r[0]) == 0, r[0]
+        return r[1] if len(r) > 1 else None
+
+    def tensor(self, i, like):
+        """A bf16 tensor over buffer i with the values of `like`."""
+        class Raw:
+            __cuda_array_interface__ = {"shape": tuple(like.shape), "typestr": "<i2", "data": (self.at[i], False), "version": 3}
+        t = torch.as_tensor(Raw(), device="cuda").view(torch.bfloat16)
+        t.copy_(like)
+        return t
+
+    def free(self):
+        torch.cuda.synchronize()
+        for a, h in zip(self.at, self.handles):
+            self.ok(self.cu.cuMemUnmap(a, self.size))
+            self.ok(self.cu.cuMemRelease(h))
+        self.ok(self.cu.cuMemAddressFree(self.base, self.total))
+
+
+@pytest.mark.parametrize("where", ["far", "far, up first", "same"])
+@pytest.mark.parametrize("H,Is,T", [(64, 64, 70), (320, 448, 300)])
+def test_shared_matrices_that_one_map_cannot_span(lib, where, H, Is, T):
+    """The gate and up matrices of a shared expert further apart than a tensor map's stride reaches (or one and the
+    same): still on the tensor cores, bit-equal to matrices that lie together."""
+    model = TinyModel(seed=T + Is, L=1, E=4, H=H, I=64, k=2, shared_I=Is)
+    wg, wu, wd = (dev_bf16(m) for m in model.shared[0])
+    if where == "same":
+        wu = wg.clone()
+    x, ys = dev_bf16(model.hidden_stream(T, 1)[0]), []
+    far = FarPair(wg.numel() * 2)
+    for split in (False, True):
+        if not split:
+            shared = [wg, wu, wd]
+        elif where == "same":
+            shared = [wg, wg, wd]
+        else:
+            order = (1, 0) if where == "far, up first" else (0, 1)
+            shared = [far.tensor(order[0], wg), far.tensor(order[1], wu), wd]
+        cache = model.make_cache(cache_rate=1.0, num_predict_expert_per_layer=0)
+        cache.set_layer_weights(0, dev_bf16(model.gate_w[0]), model.I, 2, False, gate_bias=torch.from_numpy(model.gate_bias[0]).cuda(),
+                                shared=shared)
+        ys.append(cache.forward(0, x).clone())
+        assert cache.get("tc_error") == "0" and int(cache.get("tc_launches")) > 0
+        cache.close()
+    far.free()
+    assert torch.equal(ys[0], ys[1])
+    model.shared[0] = (model.shared[0][0], model.shared[0][0] if where == "same" else model.shared[0][1], model.shared[0][2])
+    ref, _, _ = model.oracle_forward(0, x.float().cpu().numpy())
+    assert np.linalg.norm(ys[1].float().cpu().numpy() - ref) / np.linalg.norm(ref) < 8e-3
