@@ -215,8 +215,9 @@ int pm_moe_forward(pm_ctx* ctx, int layer, const void* x_dev, int T, void* y_dev
  * pm_moe_forward; there is no router, no shared expert and no combine (gate_w of the layer may be
  * NULL). An id outside [-1, num_expert) is PM_ERR_INVALID. max_rows_per_expert (0 = unknown) is a
  * bound on the rows one expert can receive that the caller guarantees, e.g. the number of tokens
- * in flight on all ranks: up to 16, the resident experts start before the host has read the row
- * counts. pred_scores (device f32 [n_pred, pred_width], may be NULL) are predictor scores for the
+ * in flight on all ranks: up to 32 the resident experts start before the host has read the row
+ * counts (uint4 experts: for up to 8 rows per expert on average, with or without a bound). A bound
+ * below the truth costs time, not correctness. pred_scores (device f32 [n_pred, pred_width], may be NULL) are predictor scores for the
  * layers pred_layers[0..n_pred) (host int32) over the pred_width experts of the WHOLE model, of
  * which this context holds [pred_first, pred_first + num_expert): the pred_top best of the whole
  * list are taken (descending score, ties to the lower id) and those among them that this context

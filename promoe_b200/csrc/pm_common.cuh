@@ -147,6 +147,7 @@ int plan_groups_size(const pm_ffn_group* groups, int n_groups, int hidden, FfnPl
 constexpr int kMaxSharedSlices = 8;
 constexpr int kMaxFusedGroups = 256 + kMaxSharedSlices;  // groups of one fused launch
 constexpr int kMaxFusedGroupsQ4 = 128;                    // same for uint4 experts (larger table records)
+inline __host__ __device__ constexpr int fused_table_size(int quant4) { return quant4 ? kMaxFusedGroupsQ4 : kMaxFusedGroups; }
 
 // What the fused kernel needs to describe, on the device, the shared expert and the routed experts
 // a layer's slot table shows resident (no host round trip between the router and this launch).
@@ -172,13 +173,21 @@ struct ResidentArgs {
 // or the one for 16. uint4: chunks of 8, the unpacking limits that kernel and its 16-row variant takes 1.6
 // times as long per chunk, so an expert of 9-16 rows (unpacked twice) is the smaller cost.
 inline int resident_chunk_rows(int row_bound, int quant4) { return quant4 || row_bound <= 8 ? 8 : 16; }
-// Most chunks such a launch can have.
+// Chunks of an expert with `rows` rows (0: left out).
+inline __host__ __device__ int resident_chunks(const ResidentArgs& a, int rows) {
+  return rows <= a.max_rows ? (rows + a.chunk_rows - 1) / a.chunk_rows : 0;
+}
+// Chunks of the shared expert: slices of its width, each over all tokens.
+inline __host__ __device__ int resident_shared_chunks(const ResidentArgs& a) {
+  return a.shared_inter > 0 ? (a.shared_inter + a.shared_slice - 1) / a.shared_slice * ((a.tokens + a.chunk_rows - 1) / a.chunk_rows) : 0;
+}
+// Most chunks such a launch can have if no expert has more than row_bound rows. A caller's bound may be wrong: a launch
+// whose chunks do not fit the table does nothing, and the host, which counts them as the kernel does, plans it all.
 inline int resident_max_chunks(const ResidentArgs& a, int row_bound) {
   const int most = row_bound < a.max_rows ? row_bound : a.max_rows;
   const int per = (most + a.chunk_rows - 1) / a.chunk_rows;
   const int routed = a.n_routed_rows / a.chunk_rows + a.num_expert;
-  const int slices = a.shared_inter > 0 ? (a.shared_inter + a.shared_slice - 1) / a.shared_slice : 0;
-  return (routed < per * a.num_expert ? routed : per * a.num_expert) + slices * ((a.tokens + a.chunk_rows - 1) / a.chunk_rows);
+  return (routed < per * a.num_expert ? routed : per * a.num_expert) + resident_shared_chunks(a);
 }
 // Width of one slice of a shared expert of width shared_inter beside routed experts of width inter.
 inline int shared_slice_width(int inter, int shared_inter) {
@@ -195,8 +204,8 @@ inline int shared_slice_count(int inter, int shared_inter) {
 }
 // Launches the fused FFN for the shared expert (sliced) and every activated resident expert.
 // counters: kMaxFusedGroups + 1 int32 (per chunk, then the launch total), zero at launch. err: a device word that receives a non-zero
-// code if a bounded dependency wait gives up. Needs cooperative launch and resident_max_chunks within the kernel's
-// table (kMaxFusedGroups, uint4: kMaxFusedGroupsQ4).
+// code if a bounded dependency wait gives up. Needs cooperative launch; does nothing where the chunks exceed the kernel's
+// table (fused_table_size).
 cudaError_t launch_resident_ffn(const ResidentArgs& a, int32_t* counters, int32_t* err,
                                 const __nv_bfloat16* x, int hidden, const int32_t* row_token,
                                 __nv_bfloat16* hbuf, int ld_h, float* yexp, cudaStream_t s);

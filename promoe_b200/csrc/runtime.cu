@@ -893,7 +893,7 @@ DevicePlan choose_device_plan(pm_ctx* c, int layer, const pm_layer_weights& w, b
   a->max_rows = w.quant4 && tc_ok ? kQ4TcMinRows - 1 : R;
   const bool tc = tc_ok && (w.quant4 ? !routed && R >= kQ4TcMinRows * E : bf16_call_on_tc(has_shared, routed, R, E, row_bound, 0));
   if (split && resident_ffn_available(a->chunk_rows, w.quant4) &&
-      resident_max_chunks(*a, row_bound) <= (w.quant4 ? kMaxFusedGroupsQ4 : kMaxFusedGroups))
+      resident_max_chunks(*a, row_bound) <= fused_table_size(w.quant4))
     return DevicePlan::kSplit;
   return tc ? DevicePlan::kTc : DevicePlan::kNone;
 }
@@ -940,7 +940,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   const int row_bound = (routed && routed->max_rows_per_expert > 0) ? std::min(T, routed->max_rows_per_expert) : T;
   ResidentArgs res{};
   const DevicePlan plan = choose_device_plan(c, layer, w, has_shared, sliced, routed != nullptr, T, R, row_bound, &res);
-  const bool spec = plan != DevicePlan::kNone;
+  bool spec = plan != DevicePlan::kNone;
   int32_t* zero_words = plan == DevicePlan::kSplit ? c->d_res_counters : nullptr;
   if (!routed && route_small_usable(T, H)) {
     RouteArgs a{};
@@ -1126,9 +1126,15 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   if (can_evict)
     for (int e = 0; e < E; ++e)
       if (resident_line[e] >= 0 && counts[e] == 0) c->line_read[resident_line[e]] = read_before[e];
-  if (spec)  // experts the device-planned launch left out
+  if (plan == DevicePlan::kSplit) {  // a row bound below the truth: the launch found no room for its chunks and did nothing
+    int chunks = resident_shared_chunks(res);
     for (int e = 0; e < E; ++e)
-      if (plan == DevicePlan::kTc ? w.quant4 && counts[e] < kQ4TcMinRows : counts[e] > res.max_rows) resident_line[e] = -1;
+      if (resident_line[e] >= 0) chunks += resident_chunks(res, counts[e]);
+    spec = chunks <= fused_table_size(w.quant4);
+  }
+  if (plan != DevicePlan::kNone)  // experts the device-planned launch left out
+    for (int e = 0; e < E; ++e)
+      if (!spec || (plan == DevicePlan::kTc ? w.quant4 && counts[e] < kQ4TcMinRows : counts[e] > res.max_rows)) resident_line[e] = -1;
   if (keep) {
     c->last_ids[layer].assign(st.ids, st.ids + R);
     c->last_w[layer].assign(st.w, st.w + R);
@@ -1166,7 +1172,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   }
   rt_mark_dirty(c, acts);
 
-  if (spec && (c->profile_ffn || (plan == DevicePlan::kTc && w.quant4))) {
+  if (plan != DevicePlan::kNone && (c->profile_ffn || (plan == DevicePlan::kTc && w.quant4))) {
     int64_t n_res = 0;
     for (int e = 0; e < E; ++e)
       if (counts[e] > 0 && resident_line[e] >= 0) ++n_res;

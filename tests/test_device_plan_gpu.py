@@ -5,8 +5,10 @@ import numpy as np
 import pytest
 import torch
 
+from oracle import moe_math as om
 from oracle import quant4 as oq
 from oracle import srs_policy as sp
+from promoe_b200 import _lib
 from promoe_b200 import quant4 as pq
 from promoe_b200.engine import ExpertCache
 from tests.helpers import TinyModel, dev, dev_bf16
@@ -89,3 +91,38 @@ def test_outputs_do_not_depend_on_what_the_cache_held(lib, kind, T):
         assert cache.get("tc_error") == "0"
         cache.close()
     assert all(torch.equal(ys[0], y) for y in ys[1:])
+
+
+# the chunks of the real rows against the kernel's table (264, uint4 128): fit; do not fit, with rows for the tensor cores and
+# without; do not fit, uint4
+@pytest.mark.parametrize("E,rows,bound,quant4", [(8, 20, 4, False), (64, 36, 8, False), (128, 30, 8, False), (100, 9, 1, True),
+                                                 (8, 32, 32, False)])
+def test_row_bound_below_the_truth_costs_no_row(lib, E, rows, bound, quant4):
+    H = I = 128 if quant4 else 64
+    model = TinyModel(seed=E + rows, L=1, E=E, H=H, I=I, k=1)
+    n = min(E * rows, 8 * E if quant4 else E * rows)
+    if quant4:
+        cache = q4_model_cache(model, 1.0)
+        mats = [[oq.dequantize(model.raw[0][e][2 * i], model.raw[0][e][2 * i + 1]) for i in range(3)] for e in range(E)]
+    else:
+        cache, mats = model.make_cache(cache_rate=1.0, num_predict_expert_per_layer=0), model.experts[0]
+    cache.report_layer(0, list(range(E)))  # every expert is resident before the call
+    for e in range(E):
+        cache.expert_done(0, e)
+    cache.layer_done(0)
+    ids = (np.arange(n) // rows).astype(np.int32)
+    np.random.default_rng(n).shuffle(ids)
+    x = model.hidden_stream(n, 1)[0]
+    xd, idd = dev_bf16(x), dev(ids)
+    out = torch.full((n, H), float("nan"), dtype=torch.float32, device="cuda")
+    for _ in range(2):
+        _lib.call("pm_moe_forward_routed", cache.handle, 0, xd.data_ptr(), n, idd.data_ptr(), out.data_ptr(), bound, None, None,
+                  0, 0, 0, 0, None)
+        torch.cuda.synchronize()
+    assert cache.get("tc_error") == "0"
+    cache.close()
+    got = out.cpu().numpy()
+    for e in range(E):
+        if (ids == e).any():
+            ref = om.swiglu_mlp(x[ids == e], *mats[e], round_h_bf16=True)
+            np.testing.assert_allclose(got[ids == e], ref, rtol=2e-2, atol=2e-2 * np.abs(ref).max() * 0.25)
