@@ -331,8 +331,9 @@ cudaError_t launch_gate(const __nv_bfloat16* x, const __nv_bfloat16* w_gate, con
   const int warps = std::min(kMaxGateThreads / 32, (n_rows + EPW - 1) / EPW);
   const size_t smem = (size_t)TOK * H * 2;
   auto kern = gate_topk_kernel<TOK, EPW, UNROLL>;
+  static SmemOptIn once;
   if (smem > 32 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = opt_in_smem(once, kern);
     if (e != cudaSuccess) return e;
   }
   return launch_behind(kern, (T + TOK - 1) / TOK, warps * 32, smem, s, x, w_gate, bias, w_shared_gate, T, H, E, k, norm_topk,
@@ -348,8 +349,9 @@ bool route_small_usable(int T, int H) { return T <= kRouteMaxTokens && route_sma
 cudaError_t launch_route_small(const RouteArgs& a, cudaStream_t s) {
   const size_t smem = route_small_smem(a.T, a.H);
   auto kern = a.T > 1 ? route_small_kernel<4> : route_small_kernel<1>;
+  static SmemOptIn once[2];
   if (smem > 16 * 1024) {  // beside 19 KB of static shared memory
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = opt_in_smem(once[a.T > 1], kern);
     if (e != cudaSuccess) return e;
   }
   return launch_behind(kern, kRouteCtas, kRouteThreads, smem, s, a);

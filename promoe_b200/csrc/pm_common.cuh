@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -70,6 +71,26 @@ constexpr int kQ4TcMinRows = 64;
 // its own CTAs can be resident (a successor that waits may hold an SM). Walls of a pass, in turn on one GPU: one token
 // 45.9 -> 43.6 us, two layers of 8 tokens with predictors 208.9 -> 191.4, routed rows 48.4 -> 45.1, 777 tokens 312 -> 299.
 #ifdef __CUDACC__
+// Opts a kernel in to all the dynamic shared memory a block can have beside its static part, once per device: the limit
+// belongs to the function, so a launch that set it to its own need could take away what another thread's launch had just set.
+struct SmemOptIn {
+  std::atomic<char> done[64] = {};
+};
+template <class... P>
+cudaError_t opt_in_smem(SmemOptIn& once, void (*kern)(P...)) {
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const bool known = dev >= 0 && dev < 64;
+  if (known && once.done[dev].load(std::memory_order_acquire)) return cudaSuccess;
+  cudaFuncAttributes attr{};
+  if ((e = cudaFuncGetAttributes(&attr, kern)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)attr.sharedSizeBytes);
+  if (e == cudaSuccess && known) once.done[dev].store(1, std::memory_order_release);
+  return e;
+}
+
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>

@@ -231,8 +231,9 @@ namespace {
 cudaError_t launch_fc1(const __nv_bfloat16* x, int B, int H, const __nv_bfloat16* w1, const float* b1, int D,
                        float* hidden_scratch, cudaStream_t s) {
   const size_t fc1_smem = (size_t)kFc1Tok * H * 2;
+  static SmemOptIn once;
   if (fc1_smem > 48 * 1024) {
-    cudaError_t ae = cudaFuncSetAttribute(predictor_fc1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fc1_smem);
+    cudaError_t ae = opt_in_smem(once, predictor_fc1_kernel);
     if (ae != cudaSuccess) return ae;
   }
   return launch_behind(predictor_fc1_kernel, (D + kWarpsPerCta - 1) / kWarpsPerCta, kWarpsPerCta * 32, fc1_smem, s, x, B, H, w1,
