@@ -76,6 +76,8 @@ int pm_ctx_get(pm_ctx* ctx, const char* key, char* buf, size_t cap) {
   if (k == "keep_routing") v = ctx->keep_routing ? "true" : "false";
   else if (k == "seq_len") v = std::to_string(ctx->seq_len);
   else if (k == "tc_launches") v = std::to_string(ctx->tc_launches);
+  else if (k == "planned_split_launches") v = std::to_string(ctx->planned_split_launches);
+  else if (k == "planned_tc_launches") v = std::to_string(ctx->planned_tc_launches);
   else if (k == "q4_expanded") v = std::to_string(ctx->q4_expanded);
   else if (k == "topn_launches") v = std::to_string(ctx->topn_launches);
   else if (k == "device_topn") v = ctx->device_topn ? "1" : "0";

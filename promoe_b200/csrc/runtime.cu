@@ -1077,10 +1077,12 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
       PM_CUDA(launch_prefill_ffn(a, s, c->profile_ffn ? spec_sample.e1 : nullptr));
       c->kernel_launches += 2;
       c->tc_launches += 1;
+      c->planned_tc_launches += 1;
     } else {
       if (c->profile_ffn) PM_CUDA(cudaEventRecord(spec_sample.e0, s));
       PM_CUDA(launch_resident_ffn(res, c->d_res_counters, c->d_tc_err, x, H, c->d_row_token, c->d_hbuf, c->ws_inter, c->d_yexp, s));
       c->kernel_launches += 1;
+      c->planned_split_launches += 1;
     }
     if (c->profile_ffn) PM_CUDA(cudaEventRecord(spec_sample.e2, s));
     // Where the layer's pool has a line for every expert nothing is ever copied over a line that holds one, so nothing

@@ -145,6 +145,7 @@ struct pm_ctx {
   bool xperm_ready = false, tc_maps_ready = false;  // per layer call
   pm::TcMaps tc_maps;
   int64_t tc_launches = 0;
+  int64_t planned_split_launches = 0, planned_tc_launches = 0;  // FFN launches planned on the device, by kernel
   // device-side ranking of the predictor scores: [2 * num_layer][kTopCap] ids (own predictions by
   // target layer, then the caller-supplied score rows of the routed-rows form)
   bool device_topn = true;

@@ -1,6 +1,7 @@
 """Launches planned on the device behind the router (resident experts and the shared expert, before the host has
 read the row counts): experts with more rows than one chunk, absent experts, both kernels, against the float64
-oracle; cache log exact."""
+oracle; cache log exact. Every case says which kernel the call was planned for ("split", "tc", None = the host waits
+for the counts) and the launch counters have to agree."""
 import numpy as np
 import pytest
 import torch
@@ -16,7 +17,7 @@ from tests.helpers import TinyModel, dev, dev_bf16
 pytestmark = pytest.mark.gpu
 
 
-def check(model, cache, T, rate, n_params, rtol, steps=3):
+def check(model, cache, T, rate, n_params, rtol, plan, steps=3):
     cache.enable_event_log(True)
     oc = sp.SequentialCache(model.L, model.E, model.k, cache_rate=rate, num_predict=0, num_per_expert_param=n_params)
     for x in model.hidden_stream(T, steps):
@@ -26,21 +27,25 @@ def check(model, cache, T, rate, n_params, rtol, steps=3):
             np.testing.assert_allclose(got, ref, rtol=rtol, atol=rtol * np.abs(ref).max() * 0.25)
             assert np.linalg.norm(got - ref) / np.linalg.norm(ref) < 8e-3
     assert cache.get("tc_error") == "0"
+    for kind in ("split", "tc"):
+        assert int(cache.get(f"planned_{kind}_launches")) == (steps * model.L if plan == kind else 0)
     assert cache.events() == oc.events
     cache.close()
 
 
-# 9, 17 and 32 rows: either side of a chunk; 33 and 70: the tensor cores, one and three 32-column granules
-@pytest.mark.parametrize("T", [9, 17, 32, 33, 70])
+# 9, 17 and 32 rows: either side of a chunk; 33 and 70: one to three 32-column granules; 610: experts of several
+# token tiles (305 rows on average) and a ragged last granule
+@pytest.mark.parametrize("T,plan", [(9, "split"), (17, "split"), (32, "split"), (33, "tc"), (70, "tc"), (610, "tc")])
 @pytest.mark.parametrize("shared,rate", [(192, 1.0), (0, 1.0), (192, 0.5)])
-def test_bf16_batches(lib, T, shared, rate):
+def test_bf16_batches(lib, T, plan, shared, rate):
     model = TinyModel(seed=60 + T, L=2, E=4, H=192, I=64, k=2, shared_I=shared, shared_gate=shared > 0)
-    check(model, model.make_cache(cache_rate=rate, num_predict_expert_per_layer=0), T, rate, 3, 2e-2)
+    check(model, model.make_cache(cache_rate=rate, num_predict_expert_per_layer=0), T, rate, 3, 2e-2, plan)
 
 
-# chunks of 8 rows up to 8 rows per expert on average, then the host's plan, then the tensor cores
-@pytest.mark.parametrize("T,rate", [(3, 1.0), (16, 1.0), (16, 0.5), (30, 1.0), (60, 1.0), (60, 0.5)])
-def test_uint4_batches(lib, T, rate):
+# chunks of 8 rows up to 8 rows per expert on average, then the host's plan, from 64 rows the tensor cores
+@pytest.mark.parametrize("T,rate,plan", [(3, 1.0, "split"), (16, 1.0, "split"), (16, 0.5, "split"), (17, 1.0, None), (30, 1.0, None),
+                                         (60, 1.0, None), (60, 0.5, None), (127, 0.5, None), (128, 1.0, "tc"), (610, 1.0, "tc"), (610, 0.5, "tc")])
+def test_uint4_batches(lib, T, rate, plan):
     model = TinyModel(seed=90 + T, L=1, E=4, H=256, I=128, k=2, norm_topk=True, zipf_bias=False, gate_std=0.2)
     cache = ExpertCache(1, 4, num_expert_per_token=2, cache_rate=rate, num_predict_expert_per_layer=0)
     cache.set_param_list(["w1.qweight", "w1.scale_zero", "w3.qweight", "w3.scale_zero", "w2.qweight", "w2.scale_zero"])
@@ -55,7 +60,7 @@ def test_uint4_batches(lib, T, rate):
     cache.pin_all()
     cache.build_slab()
     cache.set_layer_weights(0, dev_bf16(model.gate_w[0]), model.I, 2, True, quant4=True)
-    check(model, cache, T, rate, 6, 3e-2)
+    check(model, cache, T, rate, 6, 3e-2, plan)
 
 
 def q4_model_cache(model, rate):
