@@ -14,7 +14,7 @@
 // traffic, about 10 TB/s out of L2, is what is left.
 //
 // Persistent: one pair per two SMs walks the tiles pair, pair + n_pairs, ... Warp 0 loads (TMA, 128-byte
-// swizzle, 6-stage mbarrier ring), one thread of the pair's first CTA issues the MMAs, and four warps per
+// swizzle, 6-stage mbarrier ring), one thread of the pair's first CTA issues the MMAs, and eight warps per
 // CTA drain the accumulators, which are double-buffered in tensor memory (2 x 256 columns) so that an
 // epilogue runs under the next tile's MMAs. Gate and up rows alternate in blocks of 16, so that a warp's
 // 32 accumulator rows are 16 gate rows and the 16 up rows that go with them: one shuffle per two columns
@@ -37,7 +37,7 @@
 // reference runs in its Python expert loop (src/sparse_llm_cache/utils/hooks.py:187-198).
 //
 // Every mbarrier wait is bounded; on a give-up the kernel records a code in *err, stops all roles of
-// the pair, frees its tensor memory and returns.
+// the CTA (the pair's other CTA runs into its own limit), frees its tensor memory and returns.
 #include <algorithm>
 
 #include "pm_common.cuh"
@@ -49,12 +49,10 @@ namespace {
 
 using namespace sm100;
 
-// Epilogue warps: one or two per quadrant of the accumulator rows.
-template <bool Q4>
-constexpr int epi_warps() { return 8; }
+constexpr int kEpiWarps = 8;      // two per quadrant of the accumulator rows
 constexpr int kDequantWarps = 8;  // uint4 experts: two threads per weight row of a stage
 template <bool Q4>
-constexpr int tc_threads() { return (4 + epi_warps<Q4>() + (Q4 ? kDequantWarps : 0)) * 32; }
+constexpr int tc_threads() { return (4 + kEpiWarps + (Q4 ? kDequantWarps : 0)) * 32; }
 // k per stage in swizzle atoms of 64 (128 bytes of bf16): one, or a whole quantisation group for uint4
 template <bool Q4>
 constexpr int tc_atoms() { return Q4 ? 2 : 1; }
@@ -233,7 +231,7 @@ prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ 
   unsigned char* raw = stages + (size_t)ring.n_stages * ring.stage_bytes;
   TcShared& sh = *reinterpret_cast<TcShared*>(raw + (size_t)ring.n_raw * kRawBytes);
   constexpr int kAtoms = tc_atoms<Q4>(), kStageK = 64 * kAtoms, kWBytes = kAtoms * kAtomBytes;
-  constexpr int kEpiWarps = epi_warps<Q4>(), kFirstDequant = 4 + kEpiWarps;
+  constexpr int kFirstDequant = 4 + kEpiWarps;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
@@ -389,9 +387,10 @@ prefill_ffn_kernel(const __grid_constant__ TcMaps maps, const __grid_constant__ 
       sh.abort = 1;
     }
   } else if (Q4 && warp >= kFirstDequant) {
-    // ---- expand: a thread turns half of one row's quantisation group (a stage) into bf16, written where TMA would have put them (128-byte swizzle). The packed words of the next
-    // stage are in registers and its barriers polled before a stage's writes are fenced, so that only
-    // the arithmetic is left on the chain from stage to stage.
+    // ---- expand: a thread turns half of one row's quantisation group (a stage) into bf16, written where TMA
+    // would have put them (128-byte swizzle). The packed words of the next stage are in registers and its
+    // barriers polled before a stage's writes are fenced, so that only the arithmetic is left on the chain from
+    // stage to stage.
     constexpr int kChunks = 16 / kDequantWarps;  // 16-byte pieces (32 weights) of packed words per thread
     const int idx = threadIdx.x - kFirstDequant * 32;
     const int row = idx & 127, part = idx >> 7;

@@ -128,7 +128,7 @@ int ensure_workspace(pm_ctx* c, int T, const pm_layer_weights& w) {
   // shared expert into up to kMaxSharedSlices slices with a row per token each
   const size_t R = (size_t)cap * k, rows = R + cap + (size_t)kSplitMaxRows * kMaxSharedSlices;
   {
-    // worst case of one layer call: every expert plus the shared expert, chunks of 64 rows, smallest
+    // worst case of one layer call: every expert plus the shared expert, chunks of 16 rows, smallest
     // tiles, and a few extra segments each aligned to 256 bytes
     FfnPlanInfo worst;
     worst.n_desc = E + (int)(rows / kSplitMaxRows) + 8 + kMaxSharedSlices;

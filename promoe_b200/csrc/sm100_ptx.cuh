@@ -126,9 +126,6 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, u
       ::"r"(smem_u32(dst)), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
       : "memory");
 }
-__device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
 
 // 4 bytes global -> shared without registers; the calling thread's copies so far arrive on `bar` when done.
 __device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
