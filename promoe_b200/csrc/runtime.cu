@@ -839,13 +839,26 @@ int finish_forward(pm_ctx* c, PendingForward& p) {
 
 namespace {
 
-// Whether the bf16 groups of a layer call run on the tensor cores: with a group of more than kSplitChunkedMaxRows
-// rows (a shared expert has T) all of them do, without a shared expert also from 16 rows per expert on average. A rule
-// on the call, not on a launch: the two kernels add in different orders, and which experts share a launch depends on
-// what the cache held. max_rows: rows of the largest expert, 0 while only the sizes are known.
-bool bf16_call_on_tc(bool has_shared, bool routed, int R, int E, int row_bound, int max_rows) {
-  if (max_rows > kSplitChunkedMaxRows) return true;
-  return !routed && row_bound > kSplitChunkedMaxRows && (has_shared || R >= 16 * E);
+// Whether the bf16 groups of a layer call run on the tensor cores. A rule on the call, not on a launch: the two kernels add
+// in different orders, and which experts share a launch depends on what the cache held. With a shared expert (T rows), and
+// without one from 16 rows per expert on average, the sizes decide (counts = nullptr: only they are known). Else the
+// largest group does; but where all groups have at most 64 rows, less than three chunks each on average and few weights
+// between them, their second reads come out of L2 and cost less than the launch pair's last rounds of CTA pairs and the
+// gathered copy of the rows. Rows of 128 / 256 tokens on 16 / 8 experts of 2048 x 1408 96 / 74 us on the tensor cores,
+// 91 / 66 us in chunks; 36 such experts (620 MB, 200 tokens) 158 and 152, 64 of them (96 tokens x top-6) 221 and 243.
+constexpr int64_t kChunkedMaxBytes = 300ll << 20;
+bool bf16_call_on_tc(const pm_layer_weights& w, bool has_shared, bool routed, int R, int E, int row_bound, const int32_t* counts) {
+  if (!routed && row_bound > kSplitChunkedMaxRows && (has_shared || R >= 16 * E)) return true;
+  if (counts == nullptr) return false;
+  int groups = 0, chunks = 0, most = 0;
+  for (int e = 0; e < E; ++e) {
+    groups += counts[e] > 0;
+    chunks += (counts[e] + kSplitMaxRows - 1) / kSplitMaxRows;
+    most = std::max(most, counts[e]);
+  }
+  if (most <= kSplitChunkedMaxRows) return false;
+  if (most > kMaxChunkRows || chunks >= 3 * groups || chunks > kMaxFusedGroups) return true;
+  return (int64_t)groups * w.inter * w.hidden * 6 > kChunkedMaxBytes;
 }
 
 // The launch for the shared expert and the experts already resident, enqueued behind the router without waiting for
@@ -891,7 +904,7 @@ DevicePlan choose_device_plan(pm_ctx* c, int layer, const pm_layer_weights& w, b
   const bool tc_ok = w.quant4 ? tc_prefill_usable_q4(c, w) : tc_prefill_usable(c, w);
   const bool split = w.quant4 ? R <= 8 * E || !tc_ok : row_bound <= kSplitChunkedMaxRows;
   a->max_rows = w.quant4 && tc_ok ? kQ4TcMinRows - 1 : R;
-  const bool tc = tc_ok && (w.quant4 ? !routed && R >= kQ4TcMinRows * E : bf16_call_on_tc(has_shared, routed, R, E, row_bound, 0));
+  const bool tc = tc_ok && (w.quant4 ? !routed && R >= kQ4TcMinRows * E : bf16_call_on_tc(w, has_shared, routed, R, E, row_bound, nullptr));
   if (split && resident_ffn_available(a->chunk_rows, w.quant4) &&
       resident_max_chunks(*a, row_bound) <= fused_table_size(w.quant4))
     return DevicePlan::kSplit;
@@ -1192,7 +1205,7 @@ int rt_forward(pm_ctx* c, int layer, const void* xv, int T, void* yv, cudaStream
   p = PendingForward();
   p.layer = layer; p.T = T; p.R = R; p.n_shared = n_shared; p.k = k; p.H = H;
   p.spec = spec; p.is_routed = routed != nullptr;
-  p.bf16_tc = bf16_call_on_tc(has_shared, routed != nullptr, R, E, row_bound, *std::max_element(counts, counts + E));
+  p.bf16_tc = bf16_call_on_tc(w, has_shared, routed != nullptr, R, E, row_bound, counts);
   p.w = w; p.x = x; p.yv = yv; p.rows_out = routed ? routed->rows_out : nullptr; p.s = s;
   p.acts = std::move(acts);
   p.ids = ids;

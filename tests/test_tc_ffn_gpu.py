@@ -66,6 +66,13 @@ def test_tile_edges(lib, H, I, counts):
     assert run_routed(lib, H, I, counts) > 0
 
 
+# up to 64 rows, less than three chunks per group and few weights: the split-K tiles; a row more on one expert, or three
+# chunks per group: the tensor cores
+@pytest.mark.parametrize("counts,tc", [([64, 5, 16, 1], False), ([33, 32, 0, 0], False), ([65, 5, 16, 1], True), ([33, 33], True)])
+def test_few_weights_stay_in_chunks(lib, counts, tc):
+    assert (run_routed(lib, 256, 192, counts) > 0) == tc
+
+
 def test_up_matrix_first_in_memory(lib):
     assert run_routed(lib, 256, 192, [70, 130, 33], names=("up_proj.weight", "down_proj.weight", "gate_proj.weight")) > 0
 
