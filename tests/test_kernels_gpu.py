@@ -65,6 +65,38 @@ def test_gate_topk_bit_exact(lib, T, H, E, k, norm):
     np.testing.assert_allclose(ss, ref_ss, rtol=1e-4, atol=1e-6)
 
 
+def test_gate_from_two_threads_with_rows_of_different_size(lib):
+    """Two threads launch the same router kernel with 40 and 64 KB of shared memory, each on a stream of its own:
+    neither may take the other's opt-in away between setting it and launching."""
+    import threading
+    T, E, k, errors, start = 300, 8, 2, [], threading.Barrier(2)
+
+    def work(H):
+        rng = np.random.default_rng(H)
+        x, wg = om.bf16_round(rng.standard_normal((T, H)).astype(np.float32)), bf16_weights(rng, (E, H))
+        xd, wd = dev_bf16(x), dev_bf16(wg)
+        ids = torch.empty((T, k), dtype=torch.int32, device="cuda")
+        w = torch.empty((T, k), dtype=torch.float32, device="cuda")
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        start.wait()
+        try:
+            for _ in range(8000):
+                _lib.call("pm_k_gate_topk", ptr(xd), ptr(wd), None, None, T, H, E, k, 0, 1.0, None, ptr(ids), ptr(w), None, None,
+                          None, stream.cuda_stream)
+            stream.synchronize()
+            assert np.array_equal(ids.cpu().numpy(), om.route(om.gate_logits_canonical(x, wg, None), k, False)[0])
+        except Exception as e:  # noqa: BLE001 - reported by the test's thread
+            errors.append((H, e))
+
+    threads = [threading.Thread(target=work, args=(H,)) for H in (5120, 8192)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+
+
 def test_gate_topk_ties_pick_lower_id(lib):
     T, H, E, k = 3, 64, 8, 3
     x = np.ones((T, H), np.float32)

@@ -249,36 +249,3 @@ def test_decode_router_bit_exact(lib, T, E, k, H, shared):
         got = y.float().cpu().numpy()
         np.testing.assert_allclose(got, ref, rtol=2e-2, atol=2e-2 * np.abs(ref).max() * 0.25)
     cache.close()
-
-
-def test_two_threads_with_token_rows_of_different_size(lib):
-    """Contexts of two threads launch the same router kernel with different shared memory sizes: neither may take
-    the other's opt-in away between setting it and launching."""
-    import threading
-    sizes, errors = [(16, 4096), (13, 1024)], []  # 128 and 32 KB of token rows
-    models = [TinyModel(seed=70 + i, L=1, E=8, H=H, I=64, k=2) for i, (_, H) in enumerate(sizes)]
-    caches = [m.make_cache(cache_rate=1.0, num_predict_expert_per_layer=0) for m in models]
-    start = threading.Barrier(2)
-
-    def work(i):
-        T, H = sizes[i]
-        stream = torch.cuda.Stream()
-        x = dev_bf16(np.random.default_rng(i).standard_normal((T, H)).astype(np.float32))
-        torch.cuda.synchronize()
-        start.wait()
-        try:
-            with torch.cuda.stream(stream):
-                for _ in range(1500):
-                    caches[i].forward(0, x)
-            stream.synchronize()
-        except Exception as e:  # noqa: BLE001 - reported by the test's thread
-            errors.append((sizes[i], e))
-
-    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
-    for t in threads:
-        t.start()
-    for t in threads:
-        t.join()
-    for c in caches:
-        c.close()
-    assert not errors
