@@ -5,13 +5,13 @@
 // are cut into equal tiles of at most 256, so little work goes to padding, and an expert with 20 rows
 // streams its weights once against a 32-column tile.
 //
-// What bounds it: many rows per expert, the operands' way from L2 to the SMs (a k-step of 64 moves 32 KB per
-// CTA for 4.2 Mflop, half of each token tile comes from the pair's other CTA); few rows, HBM (six
-// stages keep about 100 KB of weight loads in flight per SM). Measured on 8192 tokens x top-6 over 64
-// experts (hidden 2048, inter 1408) + a shared expert of 2816: gate/up 660 us = 1146 TFLOP/s, down 378 us =
-// 1000 TFLOP/s (747 and 471 us with one-CTA tiles of 128 token rows and a 2-stage ring). Without its
-// epilogue the gate/up main loop takes 621 us, with the token loads left out too 509 us: the operand
-// traffic, about 10 TB/s out of L2, is what is left.
+// What bounds it: many rows per expert, the operands' way from L2 through the ring (a k-step of 64 moves 32 KB per
+// CTA for 4.2 Mflop, half of each token tile comes from the pair's other CTA): the tensor pipe is busy 61 % (gate/up) and
+// 54 % (down) of the time, L2 at 39 % and DRAM at 33-42 % of their peaks. Few rows, HBM (six stages keep about
+// 100 KB of weight loads in flight per SM). Measured on 8192 tokens x top-6 over 64 experts (hidden 2048, inter
+// 1408) + a shared expert of 2816: gate/up 622-630 us = 1200-1216 TFLOP/s, down 364-368 us = 1026-1038 TFLOP/s (747 and
+// 471 us with one-CTA tiles of 128 token rows and a 2-stage ring). In a timing experiment the gate/up main loop took
+// 621 us without its epilogue (660 with it on that box), 509 us with the token loads left out too.
 //
 // Persistent: one pair per two SMs walks the tiles pair, pair + n_pairs, ... Warp 0 loads (TMA, 128-byte
 // swizzle, 6-stage mbarrier ring), one thread of the pair's first CTA issues the MMAs, and eight warps per
@@ -28,10 +28,12 @@
 //
 // uint4 experts (Q4): the packed matrices are read straight from the cache lines. TMA brings packed rows into a
 // ring of their own, eight warps expand each weight once per 256 token rows to bf16 ((q - zero) * scale in
-// float32, rounded once) and write it where TMA would have put it, behind a proxy fence. What bounds this
-// is the expansion, 22 instructions per 8 weights (measured: 8 experts of 4096 x 14336, gate/up 340 us at 16 to
-// 64 rows per expert, 282 us without the arithmetic; 375 + 210 us with 512 tokens x top-2, where writing a
-// bf16 copy of every expert first and reading it back took 813 us plus 630 us for the products).
+// float32, rounded once) and write it where TMA would have put it, behind a proxy fence. 8 experts of 4096 x
+// 14336, 512 tokens x top-2: gate/up 375 us, down 210 us (writing a bf16 copy of every expert first and reading it back
+// took 813 us plus 630 us for the products). What bounds this: with up to 64 rows per expert gate/up took 340 us, 282 us
+// without the expansion's arithmetic (22 instructions per 8 weights); the larger part is the packed weights'
+// way from HBM, through the two 8 KB slots that three stages for 256 columns leave. The rounding of the weights is why
+// groups of fewer than kQ4TcMinRows rows do not come here.
 //
 // It replaces, for batches with many rows per expert, the per-expert torch linears the
 // reference runs in its Python expert loop (src/sparse_llm_cache/utils/hooks.py:187-198).

@@ -58,7 +58,10 @@ constexpr int kSplitTileDn = 32;    // or 32 down rows
 // (FFN of one layer, mixed launches with the same line -> one kind): 64 tokens x top-8, experts of 1-40 rows
 // (hidden 3584, inter 2560, shared 20480) 773 -> 716 us; 100 / 200 / 400 / 777 tokens x top-4 over 60 experts
 // (2048 x 1408, shared 5632) 224 -> 204, 254 -> 228, 279 -> 247, 314 -> 269 us. With the line at 0, 32 tokens x
-// top-6 over 64 experts lose: 155 us in chunks against 177 us.
+// top-6 over 64 experts lose: 155 us in chunks against 177 us. Above it, layer calls with a shared expert, chunks / tensor
+// cores: 33, 48, 64 tokens over 64 experts of 2048 x 1408 180 / 195, 193 / 205, 210 / 205 us; over 64 of 3584 x 2560 (shared
+// 20480) 749 / 664, 804 / 700, 920 / 700; over 8 of 4096 x 4096 183 / 172, 207 / 173, 230 / 174: the second reads
+// of wide experts miss L2. (A line of its own for narrow ones, at 48, is not built.)
 constexpr int kSplitChunkedMaxRows = 32;
 // Fewest rows of a uint4 group that may run on the tensor cores. They take weights rounded to bf16 after
 // dequantisation; the split-K tiles multiply the nibbles exactly and apply scale and zero to float32 sums
@@ -69,7 +72,7 @@ constexpr int kQ4TcMinRows = 64;
 // predecessor in the stream drains (programmatic dependent launch). It has to call wait_for_predecessor before it
 // touches what earlier kernels wrote; a predecessor lets it in early with let_successor_start, in every CTA, once all
 // its own CTAs can be resident (a successor that waits may hold an SM). Walls of a pass, in turn on one GPU: one token
-// 45.9 -> 43.6 us, two layers of 8 tokens with predictors 208.9 -> 191.4, routed rows 48.4 -> 45.1, 777 tokens 312 -> 299.
+// 45.9 -> 43.6 us, two layers of 8 tokens with predictors 208.9 -> 191.4, 777 tokens 312 -> 299; routed rows gained no more than runs differ.
 #ifdef __CUDACC__
 // Opts a kernel in to all the dynamic shared memory a block can have beside its static part, once per device: the limit
 // belongs to the function, so a launch that set it to its own need could take away what another thread's launch had just set.
